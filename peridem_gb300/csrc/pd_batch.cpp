@@ -72,7 +72,7 @@ uint64_t Engine::estimate_bytes(const std::vector<HostSim> &sims, int precision,
   uint32_t bits = 10;
   while ((1ull << bits) < 2 * N) ++bits;
   const uint64_t T = 1ull << bits;
-  b += 2 * T * 4 + 3 * C * 4 + ((T + 4095) / 4096 + 1) * 4;
+  b += (2 * T + 1) * 4 + 2 * C * 4 + C * sizeof(CellRec) + ((T + 4095) / 4096 + 1) * 4;
   b += C * (cand_cap ? cand_cap : 32) * 4 + C * 2;
   return b;
 }

@@ -16,16 +16,18 @@ namespace pdg {
 
 constexpr uint32_t kNoKey = 0xFFFFFFFFu;  // node not in the cell list
 
-// Node n's current position and cell (a cell is wider than the candidate radius, so two nodes
-// within it lie in the same or adjacent cells; CandWalk computes the cell the same way).
-__device__ __forceinline__ void node_cell(const DevView &v, uint64_t n, double inv_cell, long long &cx,
-                                          long long &cy, long long &cz, double &x, double &y, double &z) {
-  x = v.pos[n] + v.disp[n];
-  y = v.pos[n + v.Ncap] + v.disp[n + v.Ncap];
-  z = v.pos[n + 2 * v.Ncap] + v.disp[n + 2 * v.Ncap];
-  cx = (long long)floor(__dmul_rn(x, inv_cell));
-  cy = (long long)floor(__dmul_rn(y, inv_cell));
-  cz = (long long)floor(__dmul_rn(z, inv_cell));
+// Node n's record in the cell list, from its current position (a cell is wider than the candidate
+// radius, so two nodes within it lie in the same or adjacent cells; CandWalk computes the cell the
+// same way).
+__device__ __forceinline__ CellRec node_cell(const DevView &v, uint64_t n, uint32_t sim) {
+  const double inv = v.sp[sim].inv_cell;
+  CellRec r;
+  r.cx = cell_coord(v.pos[n] + v.disp[n], inv, r.fx);
+  r.cy = cell_coord(v.pos[n + v.Ncap] + v.disp[n + v.Ncap], inv, r.fy);
+  r.cz = cell_coord(v.pos[n + 2 * v.Ncap] + v.disp[n + 2 * v.Ncap], inv, r.fz);
+  r.node = (uint32_t)n;
+  r.sim = sim;
+  return r;
 }
 
 // Whether this step rebuilds (one thread): the accumulated movement bound against half the
@@ -39,214 +41,154 @@ __device__ __forceinline__ uint32_t bp_decide(const DevView &v, double half_skin
   return c.rebuild;
 }
 
-// Node n's cell bucket and its slot in it (count must be zeroed).
+// Node n's cell bucket and its slot in it (count must be zeroed); its candidate list restarts
+// empty (the search writes the lists that are not).
 __device__ __forceinline__ void bp_count_node(const DevView &v, uint64_t n, uint32_t *count, uint32_t *key,
-                                              uint32_t *slot, uint32_t mask) {
+                                              uint32_t *slot, uint32_t mask, uint16_t *cand_n) {
+  cand_n[n] = 0;
   const uint32_t sim = v.S == 1 ? 0u : v.parts[v.pid[n]].sim;
   if (!v.ss[sim].active) {  // finished simulations leave the cell list
     key[n] = kNoKey;
     return;
   }
-  long long cx, cy, cz;
-  double x, y, z;
-  node_cell(v, n, v.sp[sim].inv_cell, cx, cy, cz, x, y, z);
-  const uint32_t kk = cell_hash(cx, cy, cz, sim, mask);
+  const CellRec r = node_cell(v, n, sim);
+  const uint32_t kk = (cell_row(r.cy, r.cz, sim) + r.cx) & mask;
   key[n] = kk;
   slot[n] = atomicAdd(&count[kk], 1u);
 }
 
-__device__ __forceinline__ void bp_scatter_node(uint64_t n, const uint32_t *start, const uint32_t *key,
-                                                const uint32_t *slot, uint32_t *sorted) {
+__device__ __forceinline__ void bp_scatter_node(const DevView &v, uint64_t n, const uint32_t *start,
+                                                const uint32_t *key, const uint32_t *slot, CellRec *rec) {
   if (key[n] == kNoKey) return;
-  sorted[start[key[n]] + slot[n]] = (uint32_t)n;
+  rec[start[key[n]] + slot[n]] = node_cell(v, n, v.S == 1 ? 0u : v.parts[v.pid[n]].sim);
 }
 
-// Node n's candidate list: the nodes of its simulation within the candidate radius, ascending
-// in file order.
-__device__ __forceinline__ void bp_candidates_node(const DevView &v, uint64_t n, const uint32_t *count,
-                                                   const uint32_t *start, const uint32_t *sorted, uint32_t mask,
-                                                   uint32_t *cand, uint16_t *cand_n, uint32_t cap) {
-  constexpr int kMaxCand = (int)kMaxCandCap;
-  const uint32_t sim = v.parts[v.pid[n]].sim;
-  if (!v.ss[sim].active) {
-    cand_n[n] = 0;
-    return;
-  }
-  const DevSimParams &sp = v.sp[sim];
-  long long cx, cy, cz;
-  double x, y, z;
-  node_cell(v, n, sp.inv_cell, cx, cy, cz, x, y, z);
-  uint32_t list[kMaxCand];  // file indices: the reference visits contact partners in its numbering
-  int cnt = 0;
-  bool overflow = false;
-  for (int dz = -1; dz <= 1; ++dz)
-    for (int dy = -1; dy <= 1; ++dy)
-      for (int dx = -1; dx <= 1; ++dx) {
-        uint32_t kk = cell_hash(cx + dx, cy + dy, cz + dz, sim, mask);
-        uint32_t b = start[kk], e = b + count[kk];
-        for (uint32_t it = b; it < e; ++it) {
-          uint32_t m = sorted[it];
-          if (m == n) continue;
-          if (v.parts[v.pid[m]].sim != sim) continue;
-          double mx = v.pos[m] + v.disp[m];
-          double my = v.pos[m + v.Ncap] + v.disp[m + v.Ncap];
-          double mz = v.pos[m + 2 * v.Ncap] + v.disp[m + 2 * v.Ncap];
-          double ddx = mx - x, ddy = my - y, ddz = mz - z;
-          if (ddx * ddx + ddy * ddy + ddz * ddz > sp.cand_r2) continue;
-          // insert keeping ascending file order; drop duplicates (hash collisions can make
-          // two stencil cells share a bucket)
-          const uint32_t fm = v.file_of[m];
-          int pos = cnt;
-          while (pos > 0 && list[pos - 1] > fm) --pos;
-          if (pos > 0 && list[pos - 1] == fm) continue;
-          if (cnt >= (int)cap) {
-            overflow = true;
-            break;
-          }
-          for (int q = cnt; q > pos; --q) list[q] = list[q - 1];
-          list[pos] = fm;
-          ++cnt;
+// The records of one row's three buckets around cell me.cx: entries b .. b + len - 1 of the cell
+// list, taken modulo its nact records (start[0] is 0, so a range that runs past the table's last
+// bucket goes on at record 0).
+__device__ __forceinline__ void row_range(const CellRec &me, int row, const uint32_t *start, uint32_t mask,
+                                          uint32_t nact, uint32_t &b, uint32_t &len) {
+  const int dy = row % 3 - 1, dz = row / 3 - 1;
+  const uint32_t k = (cell_row(me.cy + dy, me.cz + dz, me.sim) + me.cx - 1u) & mask;
+  b = start[k];
+  len = (k + 3 <= mask + 1 ? start[k + 3] : nact + start[k + 2 - mask]) - b;
+}
+
+// Whether record q of that row holds a candidate of me: a node of the simulation in one of the
+// row's three cells (buckets are shared by hash) within the candidate radius. Distances are taken
+// in cell edges from the positions inside the cells: their rounding, a few 2^-24, is far below the
+// 1e-5 the test is widened by, so a list holds every node within the candidate radius; the
+// consumers' exact FP64 tests decide.
+__device__ __forceinline__ bool row_hit(const CellRec &me, int row, const CellRec &q) {
+  const uint32_t dy = row % 3 - 1, dz = row / 3 - 1;
+  const int dx = (int)(q.cx - me.cx);
+  if (q.node == me.node || dx < -1 || dx > 1 || q.cy != me.cy + dy || q.cz != me.cz + dz || q.sim != me.sim)
+    return false;
+  const float x = (float)dx + (q.fx - me.fx), y = (float)(int)dy + (q.fy - me.fy), z = (float)(int)dz + (q.fz - me.fz);
+  return x * x + y * y + z * z <= 1.0f + 1e-5f;
+}
+
+// Candidate list of the node of record t: the nodes of its simulation within the candidate radius,
+// ascending in file order, by one thread. Records are taken in the cell list's order, so the
+// threads of a warp walk neighbouring cells of a row and share the sectors of the buckets and
+// records they read. The list is kept sorted as it grows (few nodes have candidates, and few).
+// Bound by the latency of the bucket loads. A whole rebuild with 27 separately hashed cells per
+// node and FP64 positions gathered per entry took 8.0 ms on crush512_4m (3.98 M nodes) and 0.62 ms
+// on a 363k-node plate; with rows of cells and 32-byte records 1.9 and 0.15 ms.
+__device__ __forceinline__ void bp_candidates_node(const DevView &v, uint64_t t, const uint32_t *start,
+                                                   const CellRec *rec, uint32_t mask, uint32_t *cand, uint16_t *cand_n,
+                                                   uint32_t cap) {
+  const uint32_t nact = start[(uint64_t)mask + 1];
+  if (t >= nact) return;
+  const CellRec me = rec[t];
+  uint32_t b[9], len[9];
+#pragma unroll
+  for (int r = 0; r < 9; ++r) row_range(me, r, start, mask, nact, b[r], len[r]);
+  uint32_t *out = cand + (uint64_t)me.node * cap;
+  uint32_t cnt = 0;
+#pragma unroll
+  for (int r = 0; r < 9; ++r)
+    for (uint32_t i = 0; i < len[r]; ++i) {
+      const uint32_t at = b[r] + i;
+      const CellRec q = rec[at < nact ? at : at - nact];
+      if (!row_hit(me, r, q)) continue;
+      if (cnt < cap) {  // insert by file index
+        const uint32_t fq = v.file_of[q.node];
+        uint32_t pos = cnt;
+        while (pos > 0 && v.file_of[out[pos - 1]] > fq) {
+          out[pos] = out[pos - 1];
+          --pos;
         }
+        out[pos] = q.node;
       }
-  if (overflow) {
+      ++cnt;
+    }
+  if (!cnt) return;
+  if (cnt > cap) {
     // more partners than the list holds: the consumers walk the cell list for this node instead
     // (CandWalk), which gives the same partners in the same order; the host grows the lists
-    cand_n[n] = kCandCells;
+    cand_n[me.node] = kCandCells;
     atomicAdd(&v.cnt->cand_cells, 1u);
   } else {
-    uint32_t *out = cand + n * cap;
-    for (int i = 0; i < cnt; ++i) out[i] = v.node_of[list[i]];
-    cand_n[n] = (uint16_t)cnt;
+    cand_n[me.node] = (uint16_t)cnt;
   }
-  if (cnt && v.xnodes) v.xnodes[atomicAdd(&v.xcount[0], 1u)] = (uint32_t)n;  // FP32 form: work list
+  if (v.xnodes) v.xnodes[atomicAdd(&v.xcount[0], 1u)] = me.node;  // FP32 form: work list
 }
 
-// Words of shared memory bp_candidates_quad takes per warp: four groups' 27 stencil buckets and
-// four gather buffers of kMaxCandCap entries plus a count.
-constexpr uint32_t kCandQuadWords = 4 * 27 + 4 * (kMaxCandCap + 1);
+// Words of shared memory bp_candidates_quad takes per warp: four gather buffers of kMaxCandCap
+// entries plus a count.
+constexpr uint32_t kCandQuadWords = 4 * (kMaxCandCap + 1);
 
-// The same lists built four nodes per warp: lane group q = lane / 8 takes node n0 + q, and its
-// lane g walks stencil cells g, g + 8, g + 16 and g + 24 (those below 27; a bucket that several
-// stencil cells of the node share through a hash collision is walked once, for its lowest cell).
-// The qualifying nodes' file indices are gathered in the group's shared buffer and ranked into
-// ascending order. Lists, overflow decisions and the work list equal bp_candidates_node's: each
-// node of the simulation is found at most once, and a list overflows exactly when more than cap
-// distinct nodes qualify. A small handle's search is a chain of dependent loads per node (its
-// position, the buckets, their entries, the entries' positions); four chains per warp run side by
-// side. All 32 lanes of the warp call it with the same n0; sh holds kCandQuadWords words.
-__device__ __forceinline__ void bp_candidates_quad(const DevView &v, uint64_t n0, uint32_t lane, const uint32_t *count,
-                                                   const uint32_t *start, const uint32_t *sorted, uint32_t mask,
-                                                   uint32_t *cand, uint16_t *cand_n, uint32_t cap, uint32_t *sh) {
+// The same lists built for four records per warp (t0 .. t0 + 3): lane g of a record's eight takes
+// row g of its nine, lane 0 the ninth as well (a row holds one or two records; loading several
+// ahead took registers from the persistent step's bond loop, cubes125 38.5 -> 39.8 us per step).
+// The candidates' file indices are gathered in the record's shared buffer and ranked into ascending
+// order. A small handle's search is a chain of dependent loads per node (its record, the buckets,
+// their records); nine short chains side by side instead of one long one. All 32 lanes of the warp
+// call it with the same t0; sh holds kCandQuadWords words.
+__device__ __forceinline__ void bp_candidates_quad(const DevView &v, uint64_t t0, uint32_t lane, const uint32_t *start,
+                                                   const CellRec *rec, uint32_t mask, uint32_t *cand, uint16_t *cand_n,
+                                                   uint32_t cap, uint32_t *sh) {
   const uint32_t q = lane >> 3, g = lane & 7u;
-  const uint64_t n = n0 + q;
-  uint32_t *cells = sh + 27 * q;                           // the group's stencil buckets
-  uint32_t *buf = sh + 4 * 27 + (kMaxCandCap + 1) * q;     // its file indices, their count last
-  const bool one_sim = v.S == 1;                           // no other simulation's nodes in a bucket
-  uint32_t sim = 0;
-  bool run = false;
-  if (n < v.N) {
-    sim = one_sim ? 0u : v.parts[v.pid[n]].sim;
-    run = v.ss[sim].active != 0;
-  }
-  long long cx = 0, cy = 0, cz = 0;
-  double x = 0.0, y = 0.0, z = 0.0, r2 = 0.0;
-  uint32_t kk[4] = {0u, 0u, 0u, 0u};
-  if (run) {
-    const DevSimParams &sp = v.sp[sim];
-    node_cell(v, n, sp.inv_cell, cx, cy, cz, x, y, z);
-    r2 = sp.cand_r2;
-#pragma unroll
-    for (uint32_t r = 0; r < 4; ++r) {
-      const uint32_t c = g + 8 * r;
-      if (c < 27) {
-        const int dx = (int)(c % 3u) - 1, dy = (int)((c / 3u) % 3u) - 1, dz = (int)(c / 9u) - 1;
-        kk[r] = cell_hash(cx + dx, cy + dy, cz + dz, sim, mask);
-        cells[c] = kk[r];
-      }
-    }
-  }
+  const uint32_t nact = start[(uint64_t)mask + 1];
+  const uint64_t t = t0 + q;
+  const bool run = t < nact;
+  uint32_t *buf = sh + (kMaxCandCap + 1) * q;  // the record's candidates (file indices), their count last
   if (g == 0) buf[kMaxCandCap] = 0;
+  const CellRec me = rec[run ? t : 0];
   __syncwarp();
   if (run) {
-    bool walk[4];
-#pragma unroll
-    for (uint32_t r = 0; r < 4; ++r) {
-      const uint32_t c = g + 8 * r;
-      walk[r] = c < 27;
-      for (uint32_t c2 = 0; c2 < c && walk[r]; ++c2) walk[r] = cells[c2] != kk[r];
-    }
-    uint32_t b[4], len[4];
-#pragma unroll
-    for (uint32_t r = 0; r < 4; ++r) {
-      b[r] = walk[r] ? start[kk[r]] : 0u;
-      len[r] = walk[r] ? count[kk[r]] : 0u;
-    }
-    // the lane's buckets as one sequence, in batches of 4 entries whose loads are all issued
-    // before their tests
-    constexpr uint32_t B = 4;
-    const uint32_t tot = len[0] + len[1] + len[2] + len[3];
-    for (uint32_t i = 0; i < tot; i += B) {
-      uint32_t m[B];
-#pragma unroll
-      for (uint32_t u = 0; u < B; ++u) {
-        uint32_t off = i + u, base = b[0];
-        if (off >= len[0]) {
-          off -= len[0];
-          base = b[1];
-          if (off >= len[1]) {
-            off -= len[1];
-            base = b[2];
-            if (off >= len[2]) {
-              off -= len[2];
-              base = b[3];
-            }
-          }
-        }
-        m[u] = i + u < tot ? sorted[base + off] : (uint32_t)n;  // n: no entry
-      }
-      bool other[B];
-#pragma unroll
-      for (uint32_t u = 0; u < B; ++u) other[u] = m[u] == n || (!one_sim && v.parts[v.pid[m[u]]].sim != sim);
-      double px[B], py[B], pz[B];
-#pragma unroll
-      for (uint32_t u = 0; u < B; ++u) {
-        px[u] = v.pos[m[u]] + v.disp[m[u]];
-        py[u] = v.pos[m[u] + v.Ncap] + v.disp[m[u] + v.Ncap];
-        pz[u] = v.pos[m[u] + 2 * v.Ncap] + v.disp[m[u] + 2 * v.Ncap];
-      }
-#pragma unroll
-      for (uint32_t u = 0; u < B; ++u) {
-        if (other[u]) continue;
-        const double ddx = px[u] - x, ddy = py[u] - y, ddz = pz[u] - z;
-        if (ddx * ddx + ddy * ddy + ddz * ddz > r2) continue;
-        const uint32_t slot = atomicAdd(&buf[kMaxCandCap], 1u);
-        if (slot < cap) buf[slot] = v.file_of[m[u]];
-      }
+    uint32_t b0, len0, b1 = 0, len1 = 0;
+    row_range(me, (int)g, start, mask, nact, b0, len0);
+    if (g == 0) row_range(me, 8, start, mask, nact, b1, len1);
+    for (uint32_t j = 0; j < len0 + len1; ++j) {
+      const bool first = j < len0;
+      const uint32_t at = first ? b0 + j : b1 + (j - len0);
+      const CellRec c = rec[at < nact ? at : at - nact];
+      if (!row_hit(me, first ? (int)g : 8, c)) continue;
+      const uint32_t slot = atomicAdd(&buf[kMaxCandCap], 1u);
+      if (slot < cap) buf[slot] = v.file_of[c.node];
     }
   }
   __syncwarp();
-  if (n < v.N) {
-    if (!run) {
-      if (g == 0) cand_n[n] = 0;
-    } else {
-      const uint32_t total = buf[kMaxCandCap];
-      if (total > cap) {
-        if (g == 0) {
-          cand_n[n] = kCandCells;
-          atomicAdd(&v.cnt->cand_cells, 1u);
-        }
-      } else {
-        uint32_t *out = cand + n * cap;
-        for (uint32_t i = g; i < total; i += 8) {
-          const uint32_t fi = buf[i];
-          uint32_t rk = 0;
-          for (uint32_t j = 0; j < total; ++j) rk += buf[j] < fi;
-          out[rk] = v.node_of[fi];
-        }
-        if (g == 0) cand_n[n] = (uint16_t)total;
+  const uint32_t total = run ? buf[kMaxCandCap] : 0u;
+  if (total) {
+    if (total > cap) {  // as bp_candidates_node
+      if (g == 0) {
+        cand_n[me.node] = kCandCells;
+        atomicAdd(&v.cnt->cand_cells, 1u);
       }
-      if (g == 0 && total && v.xnodes) v.xnodes[atomicAdd(&v.xcount[0], 1u)] = (uint32_t)n;
+    } else {
+      uint32_t *out = cand + (uint64_t)me.node * cap;
+      for (uint32_t i = g; i < total; i += 8) {
+        const uint32_t fi = buf[i];
+        uint32_t rk = 0;
+        for (uint32_t j = 0; j < total; ++j) rk += buf[j] < fi;
+        out[rk] = v.node_of[fi];
+      }
+      if (g == 0) cand_n[me.node] = (uint16_t)total;
     }
+    if (g == 0 && v.xnodes) v.xnodes[atomicAdd(&v.xcount[0], 1u)] = me.node;
   }
   __syncwarp();
 }

@@ -139,17 +139,24 @@ __device__ __forceinline__ void wall_face(double dist, int dir, D3 vel, double v
   }
 }
 
-// Bucket of a broad-phase cell (hashed cell list: cells of every simulation share one table).
-__device__ __forceinline__ uint32_t cell_hash(long long cx, long long cy, long long cz, uint32_t sim,
-                                              uint32_t mask) {
-  unsigned long long h = (unsigned long long)cx * 0x9E3779B97F4A7C15ull;
-  h ^= (unsigned long long)cy * 0xC2B2AE3D27D4EB4Full + (h << 6) + (h >> 2);
-  h ^= (unsigned long long)cz * 0x165667B19E3779F9ull + (h << 6) + (h >> 2);
-  h ^= (unsigned long long)sim * 0x27D4EB2F165667C5ull;
-  h ^= h >> 31;
-  h *= 0x7FB5D329728EA185ull;
-  h ^= h >> 27;
-  return (uint32_t)h & mask;
+// Buckets of the broad phase's cells: the cells of one row (cy, cz) of a simulation occupy
+// consecutive buckets (modulo the table), so the three cells around a node in a row are one range
+// of the cell list and a 27-cell search is nine ranges.
+__device__ __forceinline__ uint32_t cell_row(uint32_t cy, uint32_t cz, uint32_t sim) {
+  uint32_t h = cy * 0x9E3779B1u + cz * 0x85EBCA77u + sim * 0xC2B2AE3Du;
+  h ^= h >> 15;
+  h *= 0x2C1B3C6Du;
+  h ^= h >> 12;
+  h *= 0x297A2D39u;
+  return h ^ (h >> 15);
+}
+
+// A coordinate's cell (modulo 2^32) and the position inside it in cell edges; the same expression
+// wherever a cell is computed.
+__device__ __forceinline__ uint32_t cell_coord(double x, double inv_cell, float &frac) {
+  const double s = __dmul_rn(x, inv_cell), fl = floor(s);
+  frac = (float)(s - fl);
+  return (uint32_t)(long long)fl;
 }
 
 // The contact partners of node n in ascending file-order index (the order in which the
@@ -166,7 +173,7 @@ struct CandWalk {
   const uint32_t *cl;
   int nc, c;
   bool cells;
-  long long cx, cy, cz;
+  uint32_t cx, cy, cz;
   double x, y, z, r2;
   uint32_t sim;
   long long last;  // file index of the partner returned last (-1: none yet)
@@ -182,9 +189,10 @@ struct CandWalk {
       x = v.pos[n] + v.disp[n];
       y = v.pos[n + v.Ncap] + v.disp[n + v.Ncap];
       z = v.pos[n + 2 * v.Ncap] + v.disp[n + 2 * v.Ncap];
-      cx = (long long)floor(__dmul_rn(x, sp.inv_cell));  // as node_cell
-      cy = (long long)floor(__dmul_rn(y, sp.inv_cell));
-      cz = (long long)floor(__dmul_rn(z, sp.inv_cell));
+      float f;
+      cx = cell_coord(x, sp.inv_cell, f);
+      cy = cell_coord(y, sp.inv_cell, f);
+      cz = cell_coord(z, sp.inv_cell, f);
       r2 = sp.cand_r2;
     }
   }
@@ -195,11 +203,11 @@ struct CandWalk {
     for (int dz = -1; dz <= 1; ++dz)
       for (int dy = -1; dy <= 1; ++dy)
         for (int dx = -1; dx <= 1; ++dx) {
-          const uint32_t kk = cell_hash(cx + dx, cy + dy, cz + dz, sim, v.cell_mask);
-          const uint32_t b = v.cell_start[kk], e = b + v.cell_count[kk];
+          const uint32_t kk = (cell_row(cy + dy, cz + dz, sim) + cx + dx) & v.cell_mask;
+          const uint32_t b = v.cell_start[kk], e = v.cell_start[kk + 1];
           for (uint32_t it = b; it < e; ++it) {
-            const uint32_t q = v.cell_sorted[it];
-            if (q == n || v.parts[v.pid[q]].sim != sim) continue;
+            const uint32_t q = v.cell_rec[it].node;
+            if (q == n || v.cell_rec[it].sim != sim) continue;
             const uint32_t fq = v.file_of[q];
             if ((long long)fq <= last || (found && fq >= best)) continue;
             const double ddx = (v.pos[q] + v.disp[q]) - x;

@@ -133,9 +133,8 @@ DevView Engine::view(int cur) const {
   v.cand = bp_.cand;
   v.cand_n = bp_.cand_n;
   v.cand_cap = bp_.cand_cap;
-  v.cell_count = bp_.count;
   v.cell_start = bp_.start;
-  v.cell_sorted = bp_.sorted;
+  v.cell_rec = bp_.rec;
   v.cell_mask = bp_.table_bits ? (uint32_t)((1ull << bp_.table_bits) - 1) : 0u;
   v.centroid = d_centroid_;
   v.afd = d_afd_;
@@ -935,10 +934,10 @@ int Engine::alloc_and_upload() {
   const uint64_t T = 1ull << bits;
   if (bp_.cand_cap == 0) bp_.cand_cap = 32;
   PD_TRY(dalloc(this, allocs_, &bp_.count, T, err));
-  PD_TRY(dalloc(this, allocs_, &bp_.start, T, err));
+  PD_TRY(dalloc(this, allocs_, &bp_.start, T + 1, err));
   PD_TRY(dalloc(this, allocs_, &bp_.key, C, err));
   PD_TRY(dalloc(this, allocs_, &bp_.slot, C, err));
-  PD_TRY(dalloc(this, allocs_, &bp_.sorted, C, err));
+  PD_TRY(dalloc(this, allocs_, &bp_.rec, C, err));
   PD_TRY(dalloc(this, allocs_, &bp_.block_sums, (T + 4095) / 4096 + 1, err));
   if (precision_ == PD_FP32C) {
     PD_TRY(dalloc(this, allocs_, &bp_.xnodes, C, err));
@@ -1158,7 +1157,7 @@ int Engine::launch_persist_steps(uint32_t n) {
   a.start = bp_.start;
   a.key = bp_.key;
   a.slot = bp_.slot;
-  a.sorted = bp_.sorted;
+  a.rec = bp_.rec;
   a.bar = persist_ws_;
   a.sums = persist_ws_ + 2;
   a.T = 1ull << bp_.table_bits;

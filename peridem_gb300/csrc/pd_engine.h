@@ -145,6 +145,15 @@ struct __align__(32) Rec32 {
   float4 p, u;
 };
 
+// An entry of the broad phase's cell list: the node's position inside its cell (in cell edges),
+// its cell (cell coordinates modulo 2^32) and its simulation. 32 bytes, so that a candidate is
+// tested from one sector instead of the six doubles of its position.
+struct __align__(32) CellRec {
+  float fx, fy, fz;
+  uint32_t node;
+  uint32_t cx, cy, cz, sim;
+};
+
 // Everything a kernel needs, passed by value.
 struct DevView {
   uint64_t N;            // nodes
@@ -196,8 +205,10 @@ struct DevView {
   const uint32_t *cand;  // [N][cap]
   const uint16_t *cand_n;  // list length, or kCandCells: walk the cell list (the list overflowed)
   uint32_t cand_cap;
-  // the broad phase's hashed cell list (valid from one rebuild to the next)
-  const uint32_t *cell_count, *cell_start, *cell_sorted;
+  // the broad phase's hashed cell list (valid from one rebuild to the next): bucket b holds the
+  // records [cell_start[b], cell_start[b + 1])
+  const uint32_t *cell_start;
+  const CellRec *cell_rec;
   uint32_t cell_mask;
   // torque centroids [P][3]
   const double *centroid;
@@ -214,7 +225,8 @@ struct DevView {
 // Broad-phase scratch (hashed cell list).
 struct BroadPhase {
   uint32_t table_bits = 0;
-  uint32_t *count = nullptr, *start = nullptr, *key = nullptr, *slot = nullptr, *sorted = nullptr;
+  uint32_t *count = nullptr, *start = nullptr, *key = nullptr, *slot = nullptr;  // start has T + 1 entries
+  CellRec *rec = nullptr;  // the nodes of active simulations, bucket by bucket
   uint32_t *block_sums = nullptr;
   uint32_t *cand = nullptr;
   uint16_t *cand_n = nullptr;
@@ -524,9 +536,10 @@ class Engine {
   bool graphs_ok_ = false;
 };
 
-// Handles up to this many nodes search contact candidates with four nodes per warp
-// (bp_candidates_quad), larger ones with one thread per node; the lists are the same.
-constexpr uint64_t kWarpCandNodes = 1ull << 20;
+// Handles below this many nodes search contact candidates with four nodes per warp
+// (bp_candidates_quad), larger ones with one thread per node; the lists are the same. At this
+// size one thread per node already gives every SM ~27 warps, which hide the loads' latency.
+constexpr uint64_t kWarpCandNodes = 1ull << 17;
 // Handles of at least this many nodes read their state back through pinned host memory.
 constexpr uint64_t kPinnedStageNodes = 1ull << 18;
 
@@ -536,7 +549,8 @@ struct PersistArgs {
   DevView v[2];
   uint32_t cur0, nsteps;
   double half_skin;
-  uint32_t *count, *start, *key, *slot, *sorted;
+  uint32_t *count, *start, *key, *slot;
+  CellRec *rec;
   uint32_t *sums;  // [grid] scan scratch
   uint32_t *bar;   // barrier arrival and release counters, zero at launch
   uint64_t T;

@@ -1248,7 +1248,10 @@ __device__ __forceinline__ bool persist_scan(const PersistArgs &a, GridBarrier &
     const uint32_t x = i < hi ? a.count[i] : 0u;
     uint32_t tot;
     const uint32_t incl = block_incl_scan(x, sh, &tot);
-    if (i < hi) a.start[i] = o + incl - x;
+    if (i < hi) {
+      a.start[i] = o + incl - x;
+      if (i + 1 == a.T) a.start[a.T] = o + incl;  // the end of the last bucket
+    }
     o += tot;
   }
   return true;
@@ -1280,16 +1283,15 @@ __global__ void __launch_bounds__(kPersistThreads, 1) k_persist(const __grid_con
       if (gtid == 0 && v.xcount) v.xcount[0] = 0;
       for (uint64_t i = gtid; i < a.T; i += gsize) a.count[i] = 0;
       if (!bar.sync()) return;
-      for (uint64_t n = gtid; n < v.N; n += gsize) bp_count_node(v, n, a.count, a.key, a.slot, a.mask);
+      for (uint64_t n = gtid; n < v.N; n += gsize) bp_count_node(v, n, a.count, a.key, a.slot, a.mask, a.cand_n);
       if (!bar.sync()) return;
       if (!persist_scan(a, bar) || !bar.sync()) return;
-      for (uint64_t n = gtid; n < v.N; n += gsize) bp_scatter_node(n, a.start, a.key, a.slot, a.sorted);
+      for (uint64_t n = gtid; n < v.N; n += gsize) bp_scatter_node(v, n, a.start, a.key, a.slot, a.rec);
       if (!bar.sync()) return;
       {  // four nodes per warp
         __shared__ uint32_t csh[kPersistThreads / 32][kCandQuadWords];
         for (uint64_t w = gwarp; w * 4 < v.N; w += nwarps)
-          bp_candidates_quad(v, w * 4, lane, a.count, a.start, a.sorted, a.mask, a.cand, a.cand_n, a.cap,
-                             csh[threadIdx.x >> 5]);
+          bp_candidates_quad(v, w * 4, lane, a.start, a.rec, a.mask, a.cand, a.cand_n, a.cap, csh[threadIdx.x >> 5]);
       }
       if (!bar.sync()) return;
     }
