@@ -580,12 +580,12 @@ def ours(args):
         serving = serving_run(args)
 
     # our kernels per step: k_bp_decide, k_extra32 (unless fused into the bond kernel: variants
-    # 6-9, 14-16 and 19), the bond kernel, k_end_step; the 7 broad-phase kernels run only in
+    # 6-9, 12-16 and 19), the bond kernel, k_end_step; the 6 broad-phase kernels run only in
     # rebuild steps when the step graph holds them in a conditional node, else every step
     # (exiting at once unless due)
-    fused = 6 <= variant <= 9 or 14 <= variant <= 16 or variant == 19 or variant >= 21
+    fused = 6 <= variant <= 9 or 12 <= variant <= 16 or variant == 19 or variant >= 21
     per_step = 3 if fused else 4
-    bp = 7 * (sim.rebuilds_timed if graph_mode == 2 else K)
+    bp = 6 * (sim.rebuilds_timed if graph_mode == 2 else K)
     # the persistent step: one cooperative launch per pd_step call of up to 1024 steps
     gpu_launches = -(-K // 1024) if graph_mode == 3 else per_step * K + bp
     line = {

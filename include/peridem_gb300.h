@@ -47,8 +47,7 @@ extern "C" {
                                      its list holds takes them from the cell list (same
                                      results) and the lists grow at the next pd_step      */
 #define PD_DERR_CONTACT_OVERFLOW 4u /* more in-range contacts than the per-node cap   */
-#define PD_DERR_STAGE_TIMEOUT 8u    /* a shared-memory staging copy missed its wait limit
-                                       (the block used global loads; results unaffected) */
+#define PD_DERR_STAGE_TIMEOUT 8u    /* not raised                                       */
 #define PD_DERR_BARRIER_TIMEOUT 16u /* a block of the persistent step (launch mode 3) waited
                                        longer than 2 s at a grid barrier; the launch stopped
                                        there and the state is not a step boundary's */

@@ -27,6 +27,7 @@ UNITS = [
     ("pd_kernels.cu", ["-fmad=false"]),
     ("pd_broadphase.cu", []),
     ("pd_fp32c.cu", []),
+    ("pd_tile.cu", []),
     ("pd_noalloc.cu", []),
     ("pd_pairs.cu", ["-fmad=false"]),
     ("pd_sell.cu", []),

@@ -43,14 +43,14 @@ uint64_t Engine::estimate_bytes(const std::vector<HostSim> &sims, int precision,
   }
   const uint64_t C = up32(N), nsl = C / 32;
   std::vector<uint32_t> file_of, node_of, deg_file;
-  order_nodes(sims, file_of, node_of, deg_file, bad, nullptr, order_bin(precision));
+  order_nodes(sims, file_of, node_of, deg_file, bad, nullptr, precision);
   std::vector<uint32_t> deg(C, 0);
   for (uint64_t n = 0; n < N; ++n) deg[n] = deg_file[file_of[n]];
   uint64_t E = 0;
   for (uint64_t sl = 0; sl < nsl; ++sl) {
     uint32_t w = 0;
     for (int l = 0; l < 32; ++l) w = std::max(w, deg[sl * 32 + l]);
-    E += 32ull * w;
+    E += 32ull * ((w + row_pad(precision) - 1) / row_pad(precision) * row_pad(precision));
   }
   uint64_t b = 0;
   // bonds
@@ -65,7 +65,8 @@ uint64_t Engine::estimate_bytes(const std::vector<HostSim> &sims, int precision,
     b += 3 * atleast1(E) * 8 + 2 * atleast1(E) * 8;
   } else {
     b += 2 * C * 32 + 3 * C * 8 + 2 * 3 * P * 8 + C + 3 * C * 8 + C + 2 * 6 * P * 4;
-    b += 2 * 4 * atleast1((N + kStageNodes - 1) / kStageNodes);  // staged-kernel record ranges
+    const uint64_t nt = (N + kTileNodes - 1) / kTileNodes;
+    if (N >= kTileMinNodes) b += nt * kTileRecords * 4 + nt * 4 + atleast1(E) * 2;  // tile arrays
     b += C * 4 + atleast1(P) * 4 + 2 * 4;                          // non-bond work lists
   }
   // broad phase
@@ -182,6 +183,11 @@ namespace {
 constexpr uint32_t kCkptMagic = 0x4B434450u;  // "PDCK"
 constexpr uint32_t kCkptVersion = 1;
 
+// A node record in a checkpoint.
+struct CkptRec {
+  float px, py, pz, w, ux, uy, uz, pad;
+};
+
 struct CkptHeader {
   uint32_t magic, version;
   int32_t precision, flags;  // flags: 1 pos saved (reset_partzero_y), 2 afd saved, 4 clamped disp
@@ -236,6 +242,27 @@ int ckpt_flags(const DevSimParams &sp, bool fused, uint64_t ncl) {
 }
 }  // namespace
 
+// Node order of a checkpoint (at[i]: the engine index, relative to the simulation's first node, of the
+// checkpoint's i-th node): the nodes of each particle in windows of kOrderWindow of the file's order,
+// by descending bond count (FP32 form: count / 16), whatever order the engine keeps them in.
+std::vector<uint32_t> Engine::ckpt_order(uint32_t sim) const {
+  const uint64_t n0 = sim_node0_[sim], nn = sim_node0_[sim + 1] - n0;
+  const uint32_t bin = precision_ == PD_FP32C ? 16u : 1u;
+  std::vector<uint32_t> at(nn);
+  const HostSim &s = sims_[sim];
+  parallel_items(s.np, [&](uint64_t p) {
+    for (uint64_t w0 = s.node_offset[p]; w0 < s.node_offset[p + 1]; w0 += kOrderWindow) {
+      const uint64_t w1 = std::min<uint64_t>(s.node_offset[p + 1], w0 + kOrderWindow);
+      for (uint64_t f = w0; f < w1; ++f) at[f] = (uint32_t)(node_of_[n0 + f] - n0);
+      std::vector<std::pair<uint32_t, uint32_t>> byc;  // (count bin, engine index)
+      for (uint64_t f = w0; f < w1; ++f) byc.push_back({h_deg_[n0 + at[f]] / bin, at[f]});
+      std::stable_sort(byc.begin(), byc.end(), [](const auto &a, const auto &b) { return a.first > b.first; });
+      for (uint64_t f = w0; f < w1; ++f) at[f] = byc[f - w0].second;
+    }
+  });
+  return at;
+}
+
 int Engine::save_sim(uint32_t sim, std::vector<uint8_t> &out) {
   if (sim >= S_) {
     err = "simulation index out of range";
@@ -270,13 +297,16 @@ int Engine::save_sim(uint32_t sim, std::vector<uint8_t> &out) {
   out.clear();
   Writer w{out};
   w.put(&h, sizeof(h));
-  std::vector<double> buf(3 * nn);
-  auto node3 = [&](const double *d) -> int {  // [3][Ncap] slice, engine order
+  std::vector<double> buf(3 * nn), rows(3 * nn);
+  const std::vector<uint32_t> at = ckpt_order(sim);
+  auto node3 = [&](const double *d) -> int {  // [3][Ncap] slice, checkpoint order
     for (int c = 0; c < 3; ++c)
       PD_TRY(check(cudaMemcpyAsync(buf.data() + c * nn, d + c * Ncap_ + n0, nn * 8, cudaMemcpyDeviceToHost, stream_),
                    "save"));
     PD_TRY(check(cudaStreamSynchronize(stream_), "save"));
-    w.put(buf.data(), 3 * nn * 8);
+    for (int c = 0; c < 3; ++c)
+      for (uint64_t i = 0; i < nn; ++i) rows[c * nn + i] = buf[c * nn + at[i]];
+    w.put(rows.data(), 3 * nn * 8);
     return PD_OK;
   };
   PD_TRY(node3(fused ? d_dispb_[cur_ ^ 1] : d_disp_));  // the completed step
@@ -289,7 +319,12 @@ int Engine::save_sim(uint32_t sim, std::vector<uint8_t> &out) {
   if (fused) {
     std::vector<Rec32> r(nn);
     PD_TRY(cpy(r.data(), d_rec_[cur_] + n0, nn * sizeof(Rec32), "save records"));
-    w.put(r.data(), nn * sizeof(Rec32));
+    std::vector<CkptRec> cr(nn);
+    for (uint64_t i = 0; i < nn; ++i) {
+      const Rec32 &x = r[at[i]];
+      cr[i] = CkptRec{x.px, x.py, x.pz, x.w, x.ux, x.uy, x.uz, 0.f};
+    }
+    w.put(cr.data(), nn * sizeof(CkptRec));
   }
   std::vector<DevPart> parts(np);
   PD_TRY(cpy(parts.data(), d_parts_ + p0, np * sizeof(DevPart), "save particles"));
@@ -368,9 +403,12 @@ int Engine::load_sim(uint32_t sim, const uint8_t *buf, uint64_t n) {
     err = "checkpoint of another setup, config or precision form than simulation " + std::to_string(sim);
     return PD_EINVAL;
   }
-  std::vector<double> nodebuf(3 * nn);
+  std::vector<double> nodebuf(3 * nn), rows(3 * nn);
+  const std::vector<uint32_t> at = ckpt_order(sim);
   auto node3 = [&](double *d) -> int {
-    if (!r.get(nodebuf.data(), 3 * nn * 8)) return PD_EINVAL;
+    if (!r.get(rows.data(), 3 * nn * 8)) return PD_EINVAL;
+    for (int c = 0; c < 3; ++c)
+      for (uint64_t i = 0; i < nn; ++i) nodebuf[c * nn + at[i]] = rows[c * nn + i];
     for (int c = 0; c < 3; ++c)
       PD_TRY(check(cudaMemcpyAsync(d + c * Ncap_ + n0, nodebuf.data() + c * nn, nn * 8, cudaMemcpyHostToDevice,
                                    stream_), "load"));
@@ -393,8 +431,14 @@ int Engine::load_sim(uint32_t sim, const uint8_t *buf, uint64_t n) {
   if ((rc = node3(d_force_)) != PD_OK) return rc == PD_EINVAL ? bad() : rc;
   if ((h.flags & 1) && (rc = node3(d_pos_)) != PD_OK) return rc == PD_EINVAL ? bad() : rc;
   if ((h.flags & 2) && (rc = node3(d_afd_)) != PD_OK) return rc == PD_EINVAL ? bad() : rc;
-  if (fused && (rc = take(d_rec_[cur_] + n0, nn * sizeof(Rec32), "load records")) != PD_OK)
-    return rc == PD_EINVAL ? bad() : rc;
+  if (fused) {
+    std::vector<CkptRec> cr(nn);
+    if (!r.get(cr.data(), nn * sizeof(CkptRec))) return bad();
+    std::vector<Rec32> x(nn);
+    for (uint64_t i = 0; i < nn; ++i)
+      x[at[i]] = Rec32{cr[i].px, cr[i].py, cr[i].ux, cr[i].uy, cr[i].pz, cr[i].uz, cr[i].w, 0.f};
+    PD_TRY(cpy(d_rec_[cur_] + n0, x.data(), nn * sizeof(Rec32), "load records"));
+  }
   if ((rc = take(d_lrtb_ + 6ull * p0, 6 * np * 8, "load boxes")) != PD_OK) return rc == PD_EINVAL ? bad() : rc;
   if (fused) {
     if ((rc = take(d_anchor_ + 3ull * p0, 3 * np * 8, "load anchors")) != PD_OK) return rc == PD_EINVAL ? bad() : rc;

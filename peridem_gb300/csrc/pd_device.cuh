@@ -267,6 +267,32 @@ __device__ __forceinline__ bool nonfinite(double x) {
   return ((__double2hiint(x) >> 20) & 0x7FF) == 0x7FF;
 }
 
+// Conversions between float and double by integer operations, exact and correctly rounded as the
+// conversion instructions are. GB300's conversions run on the FP64 pipe, 16 cycles of an SM a warp;
+// the ten or so integer instructions take 5, and a 64-cycle latency goes with them.
+// A float that is zero or normal; the other kinds take the instruction.
+__device__ __forceinline__ bool odd_float(float x) {
+  const uint32_t m = __float_as_uint(x) & 0x7FFFFFFFu;
+  return m != 0 && m - 0x00800000u >= 0x7F000000u;
+}
+__device__ __forceinline__ double widen(float x) {  // x not odd_float
+  const uint32_t b = __float_as_uint(x), m = b & 0x7FFFFFFFu;
+  return __hiloint2double((int)((b & 0x80000000u) | (m ? (m >> 3) + 0x38000000u : 0u)), (int)(b << 29));
+}
+__device__ __forceinline__ float narrow(double x) {  // round to nearest even
+  const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x), m = hi & 0x7FFFFFFFu;
+  if ((m | lo) == 0) return __uint_as_float(hi);           // +-0
+  if (m - 0x38100000u >= 0x0FD00000u) return (float)x;     // below 2^-126, from 2^127 on, or not finite
+  const uint64_t r = (((uint64_t)m << 32) | lo) + 0x0FFFFFFFu + ((lo >> 29) & 1u);  // carries into the exponent
+  return __uint_as_float((hi & 0x80000000u) | ((uint32_t)(r >> 29) - 0xC0000000u));
+}
+// |x| as a float, truncated to 20 bits of mantissa (a relative error below 2^-20; clamped to the
+// normal range): for bounds.
+__device__ __forceinline__ float magnitude(double x) {
+  const int e = (int)((uint32_t)__double2hiint(x) & 0x7FFFFFFFu) - 0x38000000;
+  return __uint_as_float((uint32_t)min(max(e, 0), 0x0FEFFFFF) << 3);
+}
+
 // FP32 form: the band [snot (1 - w), snot (1 + w)] in which a bond's breaking decision is
 // re-taken in FP64 (outside it the FP32 stretch decides), wide enough that the FP32 stretch can
 // never be on the other side of snot outside it. With eps = 2^-24 and s <= 2 snot near the band:
@@ -365,43 +391,6 @@ __device__ __forceinline__ void end_particle_fp32c(const DevView &v, uint32_t k,
     const int c = f % 3;
     wl[f] = (float)(wall_next[f] - (e.apos[c] + e.ann[c]));
   }
-}
-
-// ---- bulk copies global -> shared with an mbarrier (cp.async.bulk) --------------------
-
-__device__ __forceinline__ uint32_t smem_addr(const void *p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count) : "memory");
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes) : "memory");
-}
-// bytes: multiple of 16; both addresses 16-byte aligned
-__device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                   smem_addr(dst)),
-               "l"(src), "r"(bytes), "r"(smem_addr(bar))
-               : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t *bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-      : "=r"(ok)
-      : "r"(smem_addr(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// Waits for phase `parity` of the barrier at most `limit` polls; false when the limit ran out.
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity, uint32_t limit) {
-  for (uint32_t it = 0; it < limit; ++it) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if (it > 32) __nanosleep(128);
-  }
-  return false;
 }
 
 }  // namespace pdg

@@ -115,9 +115,12 @@ DevView Engine::view(int cur) const {
   }
   v.break_band = 1e-4;
   v.f_extra = d_f_extra_;
-  v.win_lo = d_win_lo_;
-  v.win_cnt = d_win_cnt_;
-  v.win_max = win_max_;
+  v.tile_rec = d_tile_rec_;
+  v.tile_n = d_tile_n_;
+  v.tcol = tiles_ready_ ? d_tcol_ : nullptr;
+  v.tile_max = tile_max_;
+  v.tile_gather = tiles_gathering_;
+  v.tile_vol = tile_vol_ ? 1 : 0;
   v.xnodes = bp_.xnodes;
   v.xparts = bp_.xparts;
   v.xcount = bp_.xcount;
@@ -184,10 +187,10 @@ int Engine::init(std::vector<HostSim> &sims, int precision) {
   }
   Ncap_ = round_up(N_, 32);
   nslices_ = Ncap_ / 32;
-  // default bond-kernel variant: the autotuner's choice on small and on large handles (small
-  // handles are launch-latency bound and gain most from doing the non-bond work in the bond
-  // kernel, one launch less per step)
-  variant_ = N_ < 131072 ? 25 : 18;
+  // default bond-kernel variant, as the autotuner mostly chooses: small handles gather a group ahead
+  // and do the non-bond work in the bond kernel (one launch less per step); larger ones are tiled
+  // (alloc_and_upload goes back to 18 where the tiles' records do not fit)
+  variant_ = N_ < kTileMinNodes ? 25 : N_ < kTileSplitNodes ? 12 : 10;
   // and the step graph: on large handles the broad phase's kernels are worth skipping in
   // steps without a rebuild (a conditional node); small handles replay them, exiting at once.
   // Small FP32 handles step in persistent launches (where the handle's features allow it,
@@ -205,7 +208,7 @@ int Engine::init(std::vector<HostSim> &sims, int precision) {
   final_.assign(S_, std::vector<double>());
   {
     int64_t bad = -1;
-    order_nodes(sims_, file_of_, node_of_, deg_file_, &bad, &conn_sorted_, order_bin(precision_));
+    order_nodes(sims_, file_of_, node_of_, deg_file_, &bad, &conn_sorted_, precision_);
     if (bad >= 0) {
       err = "Connectivity index out of range in particle " + std::to_string(bad);
       return PD_EINVAL;
@@ -229,20 +232,69 @@ int Engine::init(std::vector<HostSim> &sims, int precision) {
 }
 
 
+// Sorts along (0 .. n-1 on entry) by the Morton code of each node's cell, keeping file order inside
+// a cell. Cells hold ~64 nodes of the particle's mean nodal volume; at most 1024 of them a side.
+static void morton_order(const double *pos, const double *vol, std::vector<uint32_t> &along) {
+  const uint64_t n = along.size();
+  double lo[3] = {pos[0], pos[1], pos[2]}, hi[3] = {pos[0], pos[1], pos[2]}, vsum = 0;
+  for (uint64_t k = 0; k < n; ++k) {
+    for (int c = 0; c < 3; ++c) {
+      lo[c] = std::min(lo[c], pos[3 * k + c]);
+      hi[c] = std::max(hi[c], pos[3 * k + c]);
+    }
+    vsum += vol[k];
+  }
+  const double ext = std::max(std::max(hi[0] - lo[0], hi[1] - lo[1]), hi[2] - lo[2]);
+  const double cell = std::max(std::cbrt(64.0 * vsum / (double)n), ext / 1023.0), inv = 1.0 / cell;
+  if (!(cell > 0) || !std::isfinite(inv) || !std::isfinite(ext)) return;  // no geometry to go by
+  auto spread = [](uint32_t x) {  // ten bits, two zero bits between them
+    x = (x | (x << 16)) & 0x030000FFu;
+    x = (x | (x << 8)) & 0x0300F00Fu;
+    x = (x | (x << 4)) & 0x030C30C3u;
+    return (x | (x << 2)) & 0x09249249u;
+  };
+  std::unique_ptr<uint32_t[]> key(new uint32_t[n]);
+  uint32_t all = 0;
+  for (uint64_t k = 0; k < n; ++k) {
+    uint32_t m = 0;
+    for (int c = 0; c < 3; ++c) {
+      const double q = (pos[3 * k + c] - lo[c]) * inv;
+      m |= spread(q >= 0 ? (uint32_t)std::min(q, 1023.0) : 0u) << c;
+    }
+    key[k] = m;
+    all |= m;
+  }
+  std::vector<uint32_t> to(n);
+  for (int sh = 0; sh < 30 && (all >> sh); sh += 10) {  // stable radix sort of the nodes by their keys
+    uint32_t at[1025] = {0};
+    for (uint64_t k = 0; k < n; ++k) at[((key[k] >> sh) & 1023u) + 1]++;
+    for (int d = 0; d < 1024; ++d) at[d + 1] += at[d];
+    for (uint64_t k = 0; k < n; ++k) to[at[(key[along[k]] >> sh) & 1023u]++] = along[k];
+    along.swap(to);
+  }
+}
+
 void Engine::order_nodes(const std::vector<HostSim> &sims, std::vector<uint32_t> &file_of,
                          std::vector<uint32_t> &node_of, std::vector<uint32_t> &deg_file, int64_t *bad,
-                         bool *sorted, uint32_t deg_bin) {
+                         bool *sorted, int precision) {
   // The SELL-32 layout pads every row of a slice to the slice's longest row. In file order a
   // slice mixes interior nodes (full neighbourhoods) with surface nodes (truncated ones);
   // sorting by bond count makes the rows of a slice nearly equal (crush512: padded entries
-  // 1.23x the bonds in file order, 1.03x sorted). Sorting by count / deg_bin keeps more of the
-  // file's lattice order among nodes of nearly equal counts (deg_bin 16: 1.07x padding). The sort runs inside windows of
-  // kOrderWindow consecutive nodes of a particle and is stable, so a node moves less than a
-  // window and interior nodes keep their lattice order: partners stay close in memory (a
-  // whole-particle sort of a 1.5 M-node plate made the FP32 bond kernel slower).
-  // Per-node results do not depend on the order: each node's sums keep the reference's row
-  // order, and every sequence that the reference takes in node order (contact partners,
-  // particle means) is taken in file order through node_of / file_of.
+  // 1.23x the bonds in file order, 1.03x sorted by exact counts in windows of 1024). The sort runs
+  // inside windows of consecutive nodes of a particle and is stable, so a node moves less than a
+  // window and partners stay close in memory.
+  // The FP32 form's tiled bond kernel reads each tile's distinct partner records once, so its
+  // order keeps the nodes of a tile together in space: cells of ~64 nodes along a Morton curve,
+  // counted on crush512_4m's particles 1,447 records per tile of 256 nodes at any alignment of
+  // the tiles (windows of the file order: 2,407; recursive bisection, dearer to compute: 1,412), at
+  // 1.09x padding with counts sorted in bins of 16. A particle of up to kOrderWindow nodes keeps
+  // its file order: its tiles read at most the particle's records in any order.
+  // The order depends on the particle alone (a checkpoint moves between handles), and per-node
+  // results do not depend on it: each node's sums keep the reference's row order, and every
+  // sequence that the reference takes in node order (contact partners, particle means) is taken
+  // in file order through node_of / file_of.
+  const bool spatial = precision == PD_FP32C;
+  const uint32_t deg_bin = spatial ? 16u : 1u;
   struct PartRef {
     const HostSim *s;
     uint32_t p;
@@ -280,19 +332,24 @@ void Engine::order_nodes(const std::vector<HostSim> &sims, std::vector<uint32_t>
       prev = key;
     }
     if (!srt) all_sorted = false;
-    std::vector<uint32_t> idx(nloc);
+    std::vector<uint32_t> along(nloc), idx(nloc);
+    for (uint64_t k = 0; k < nloc; ++k) along[k] = (uint32_t)k;
+    const bool along_curve = spatial && nloc > kOrderWindow;
+    const uint64_t window = along_curve ? kOrderWindow32 : kOrderWindow;
+    if (along_curve) morton_order(s.pos.data() + 3 * s.node_offset[p], s.vol.data() + s.node_offset[p], along);
     std::vector<uint32_t> hist;
-    for (uint64_t w0 = 0; w0 < nloc; w0 += kOrderWindow) {
-      const uint64_t w1 = std::min<uint64_t>(nloc, w0 + kOrderWindow);
+    for (uint64_t w0 = 0; w0 < nloc; w0 += window) {
+      const uint64_t w1 = std::min<uint64_t>(nloc, w0 + window);
+      auto bin = [&](uint64_t k) { return dg[along[k]] / deg_bin; };
       uint32_t dmax = 0;
-      for (uint64_t k = w0; k < w1; ++k) dmax = std::max(dmax, (dg[k] / deg_bin));
+      for (uint64_t k = w0; k < w1; ++k) dmax = std::max(dmax, bin(k));
       if (dmax < 4096) {  // stable counting sort by descending count
         hist.assign(dmax + 2, 0);
-        for (uint64_t k = w0; k < w1; ++k) hist[dmax - (dg[k] / deg_bin) + 1]++;
+        for (uint64_t k = w0; k < w1; ++k) hist[dmax - bin(k) + 1]++;
         for (uint32_t d = 1; d <= dmax + 1; ++d) hist[d] += hist[d - 1];
-        for (uint64_t k = w0; k < w1; ++k) idx[w0 + hist[dmax - (dg[k] / deg_bin)]++] = (uint32_t)k;
+        for (uint64_t k = w0; k < w1; ++k) idx[w0 + hist[dmax - bin(k)]++] = along[k];
       } else {
-        for (uint64_t k = w0; k < w1; ++k) idx[k] = (uint32_t)k;
+        std::copy(along.begin() + w0, along.begin() + w1, idx.begin() + w0);
         std::stable_sort(idx.begin() + w0, idx.begin() + w1, [&](uint32_t a, uint32_t b) { return dg[a] / deg_bin > dg[b] / deg_bin; });
       }
     }
@@ -418,7 +475,8 @@ int Engine::bond_counts(std::vector<uint32_t> &deg, std::vector<uint64_t> *rowpt
     for (uint64_t sl = c * 4096; sl < std::min<uint64_t>(nslices_, c * 4096 + 4096); ++sl) {
       uint32_t w = 0;
       for (int l = 0; l < 32; ++l) w = std::max(w, deg[sl * 32 + l]);
-      h_slice_ptr_[sl + 1] = 32ull * w;  // widths for now
+      const uint32_t pad = row_pad(precision_);
+      h_slice_ptr_[sl + 1] = 32ull * ((w + pad - 1) / pad * pad);  // widths for now
     }
   });
   for (uint64_t sl = 0; sl < nslices_; ++sl) h_slice_ptr_[sl + 1] += h_slice_ptr_[sl];
@@ -428,15 +486,6 @@ int Engine::bond_counts(std::vector<uint32_t> &deg, std::vector<uint64_t> *rowpt
 
 int Engine::alloc_bond_arrays() {
   const uint64_t ncol = std::max<uint64_t>(E_, 1), nmask = std::max<uint64_t>(E_ / 32, 1);
-  if (precision_ == PD_FP32C) {
-    // record ranges of the staged bond kernel: computed on the device the first time a staged
-    // variant is chosen (prepare_windows)
-    const uint64_t nb = (N_ + kStageNodes - 1) / kStageNodes;
-    PD_TRY(dalloc(this, allocs_, &d_win_lo_, nb, err));
-    PD_TRY(dalloc(this, allocs_, &d_win_cnt_, nb, err));
-    win_max_ = 0;
-    windows_ready_ = false;
-  }
   PD_TRY(dalloc(this, allocs_, &d_slice_ptr_, nslices_ + 1, err));
   PD_TRY(dalloc(this, allocs_, &d_deg_, Ncap_, err));
   PD_TRY(dalloc(this, allocs_, &d_col_, ncol, err));
@@ -534,6 +583,7 @@ int Engine::upload_bonds(SellHost &h) {
 
 int Engine::alloc_and_upload() {
   const uint64_t C = Ncap_;
+  constexpr uint64_t kChunk = 8192;  // nodes a host thread stages at a time
   // The SELL-32 bond arrays: from a sorted Connectivity they are built on the device once the
   // node arrays (node_of among them) are uploaded, the bond counts being computed on a host
   // thread meanwhile; from any other Connectivity the whole build runs on a host thread beside
@@ -591,8 +641,8 @@ int Engine::alloc_and_upload() {
     HostSim &s = sims_[si];
     const pd_config &cf = s.cfg;
     const uint64_t ns = s.node_offset[s.np];
-    parallel_items((ns + 65535) / 65536, [&](uint64_t chunk) {
-      const uint64_t k0 = chunk * 65536, k1 = std::min<uint64_t>(ns, k0 + 65536);
+    parallel_items((ns + kChunk - 1) / kChunk, [&](uint64_t chunk) {
+      const uint64_t k0 = chunk * kChunk, k1 = std::min<uint64_t>(ns, k0 + kChunk);
       uint32_t p = (uint32_t)(std::upper_bound(s.node_offset.begin(), s.node_offset.begin() + s.np + 1, k0) -
                               s.node_offset.begin() - 1);
       for (uint64_t k = k0; k < k1; ++k) {
@@ -778,6 +828,7 @@ int Engine::alloc_and_upload() {
   // centre of the particle's box (the FP32 rounding of a record grows with its distance from the
   // anchor); ext_p bounds the reference positions' rounding (set_break_band). xi_min is measured
   // on the device once the bonds are built.
+  std::atomic<bool> vol_varies(false);  // inside some particle
   parallel_items(P_, [&](uint64_t k) {
     DevPart &P = parts[k];
     double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
@@ -801,14 +852,19 @@ int Engine::alloc_and_upload() {
     }
     P.anchor = a;
     double ep = 0;
+    bool same = true;
     for (int c = 0; c < 3; ++c) P.anchor_pos[c] = pos[c * C + a];
-    for (uint64_t g = P.g0; g < (uint64_t)P.g0 + P.n; ++g)
+    for (uint64_t g = P.g0; g < (uint64_t)P.g0 + P.n; ++g) {
       for (int c = 0; c < 3; ++c) ep = std::max(ep, std::fabs(pos[c * C + g] - P.anchor_pos[c]));
+      same = same && vol[g] == vol[P.g0];
+    }
+    if (!same) vol_varies = true;
     P.ext_p = ep;
     P.xi_min = INFINITY;
     P.snot_lo32 = (float)P.snot;
     P.snot_hi32 = (float)P.snot;
   });
+  tile_vol_ = vol_varies.load();
   auto up = [&](void *d, const void *h, size_t b, const char *w) { return cpy(d, h, b, w); };
   PD_TRY(up(d_pos_, pos.get(), 3 * C * 8, "upload pos"));
   PD_TRY(up(d_disp_, disp.get(), 3 * C * 8, "upload disp"));
@@ -883,18 +939,18 @@ int Engine::alloc_and_upload() {
     PD_TRY(dalloc(this, allocs_, &d_brxin_, std::max<uint64_t>(E_, 1), err));
   } else {
     std::unique_ptr<Rec32[]> r32(new Rec32[C]);  // every entry written below
-    parallel_items((C + 65535) / 65536, [&](uint64_t chunk) {
-      for (uint64_t g = chunk * 65536; g < std::min<uint64_t>(C, chunk * 65536 + 65536); ++g) {
+    parallel_items((C + kChunk - 1) / kChunk, [&](uint64_t chunk) {
+      for (uint64_t g = chunk * kChunk; g < std::min<uint64_t>(C, (chunk + 1) * kChunk); ++g) {
         Rec32 &r = r32[g];
-        r.u = make_float4(0.f, 0.f, 0.f, 0.f);
+        r = Rec32{};
         if (g < N_) {
           const DevPart &P = parts[h_pid_[g]];
           // the bond kernels' force coefficient of this node as a partner: cnot * volume (a
           // bond's partner is in the same particle)
-          r.p = make_float4((float)(pos[g] - P.anchor_pos[0]), (float)(pos[C + g] - P.anchor_pos[1]),
-                            (float)(pos[2 * C + g] - P.anchor_pos[2]), (float)(P.cnot * vol[g]));
-        } else {
-          r.p = make_float4(0.f, 0.f, 0.f, 0.f);
+          r.px = (float)(pos[g] - P.anchor_pos[0]);
+          r.py = (float)(pos[C + g] - P.anchor_pos[1]);
+          r.pz = (float)(pos[2 * C + g] - P.anchor_pos[2]);
+          r.w = (float)(P.cnot * vol[g]);
         }
       }
     });
@@ -965,6 +1021,12 @@ int Engine::alloc_and_upload() {
     PD_TRY(rc);
     cur_ = 1;
     PD_TRY(prepare_fused(cur_));
+    if (N_ >= kTileMinNodes) {
+      PD_TRY(prepare_tiles());
+      // tiles that gather from global memory run slower than the plain kernel's: use that one where
+      // they are common (horizons far wider than three node spacings)
+      if (10ull * tiles_gathering_ > (N_ + kTileNodes - 1) / kTileNodes) variant_ = 18;
+    }
   }
   PD_TRY(check(cudaStreamSynchronize(stream_), "init sync"));
   return PD_OK;
@@ -1183,7 +1245,9 @@ int Engine::step(uint32_t nsteps) {
     uint32_t z = 0;
     PD_TRY(cpy(&d_cnt_->cand_cells, &z, 4, "reset cell-walk count"));
   }
-  if (use_persist_ && persist_eligible()) {
+  const bool persist = use_persist_ && persist_eligible();
+  PD_TRY(refresh_tiles(!persist && tile_variant()));
+  if (persist) {
     for (uint32_t done = 0; done < nsteps;) {
       const uint32_t n = std::min(nsteps - done, kPersistMaxSteps);
       PD_TRY(launch_persist_steps(n));
@@ -1546,7 +1610,7 @@ int Engine::profile(uint32_t nsteps, double *phase_ms) {
   cudaEvent_t ev[5];
   for (int i = 0; i < 5; ++i)
     if (cudaEventCreate(&ev[i]) != cudaSuccess) return check(cudaGetLastError(), "event create");
-  int rc = PD_OK;
+  int rc = refresh_tiles(tile_variant());
   for (uint32_t k = 0; k < nsteps && rc == PD_OK; ++k) {
     DevView v = view(cur_);
     cudaStream_t s = stream_;
@@ -1790,6 +1854,7 @@ int Engine::restore() {
     off += (m.second + 255) & ~(size_t)255;
   }
   if (precision_ == PD_FP32C) launch_col_flags(view(cur_), stream_);  // broken flags from the masks
+  tiles_stale_ = false;
   PD_TRY(check(cudaGetLastError(), "restore"));
   {  // the next step rebuilds the broad phase from the restored positions (results do not depend
      // on when it is rebuilt); the FP32 non-bond kernel visits every node once meanwhile
@@ -1810,18 +1875,34 @@ int Engine::restore() {
   return check(cudaStreamSynchronize(stream_), "restore");
 }
 
-int Engine::prepare_windows() {
-  if (windows_ready_ || precision_ != PD_FP32C) return PD_OK;
-  const uint64_t nb = (N_ + kStageNodes - 1) / kStageNodes;
-  launch_stage_windows(view(cur_), d_win_lo_, d_win_cnt_, stream_);
-  PD_TRY(check(cudaGetLastError(), "stage windows"));
-  std::vector<uint32_t> wcnt(nb);
-  PD_TRY(cpy(wcnt.data(), d_win_cnt_, nb * 4, "read windows"));
-  win_max_ = 0;
-  for (uint32_t c : wcnt) win_max_ = std::max(win_max_, c);
-  if (win_max_) PD_TRY(prepare_staged_kernels(win_max_ * (uint32_t)sizeof(Rec32)));
-  windows_ready_ = true;
-  graphs_ok_ = false;  // the kernels' view carries win_max
+int Engine::prepare_tiles() {
+  if (tiles_ready_ || precision_ != PD_FP32C) return PD_OK;
+  const uint64_t nt = (N_ + kTileNodes - 1) / kTileNodes;
+  if (!d_tile_rec_) PD_TRY(dalloc(this, allocs_, &d_tile_rec_, nt * kTileRecords, err));
+  if (!d_tile_n_) PD_TRY(dalloc(this, allocs_, &d_tile_n_, nt, err));
+  if (!d_tcol_) PD_TRY(dalloc(this, allocs_, &d_tcol_, std::max<uint64_t>(E_, 1), err));
+  PD_TRY(check(launch_tile_build(view(cur_), d_tile_rec_, d_tile_n_, d_tcol_, stream_), "tile build"));
+  std::vector<uint32_t> cnt(nt);
+  PD_TRY(cpy(cnt.data(), d_tile_n_, nt * 4, "read tiles"));
+  tile_max_ = 0;
+  tiles_gathering_ = 0;
+  for (uint32_t c : cnt) {
+    tile_max_ = std::max(tile_max_, c);
+    tiles_gathering_ += c == 0;
+  }
+  PD_TRY(check(prepare_tile_kernels(), "tile kernels"));
+  tiles_ready_ = true;
+  graphs_ok_ = false;  // the kernels' view carries the tiles
+  return PD_OK;
+}
+
+int Engine::refresh_tiles(bool tiled) {
+  if (!tiles_ready_) return PD_OK;
+  if (tiled && tiles_stale_) {
+    launch_col_flags(view(cur_), stream_);
+    PD_TRY(check(cudaGetLastError(), "tile flags"));
+  }
+  tiles_stale_ = !tiled;
   return PD_OK;
 }
 
@@ -1840,8 +1921,8 @@ int Engine::set_variant(int variant) {
     err = "bond kernel variant out of range";
     return PD_EINVAL;
   }
-  if (variant >= kFirstStagedVariant) PD_TRY(prepare_windows());
   variant_ = variant;
+  if (tile_variant()) PD_TRY(prepare_tiles());
   graphs_ok_ = false;
   return PD_OK;
 }
@@ -1849,7 +1930,7 @@ int Engine::set_variant(int variant) {
 int Engine::autotune(uint32_t steps_per_variant, int *chosen, double *variant_ms) {
   const int nv = precision_ == PD_FP32C ? num_bond_variants() : 1;
   if (steps_per_variant == 0) steps_per_variant = 8;
-  if (nv > kFirstStagedVariant) PD_TRY(prepare_windows());
+  if (nv > kFirstTileVariant) PD_TRY(prepare_tiles());
   PD_TRY(snapshot());
   int best = variant_;
   double best_ms = 1e300;

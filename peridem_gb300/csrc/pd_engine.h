@@ -21,9 +21,8 @@
 //     the masks stay the record every other reader uses;
 //   * FP64 form only: per-entry constants xi = pos[q]-pos[i] (3 doubles), |xi| and the
 //     correctly rounded reciprocal of |xi| (gen_xi, particle2.h:241-257);
-//   * FP32-compensated form only: a 32-byte record per node, float4 (local position,
-//     cnot * volume) + float4 (local displacement), double-buffered; local = relative to the
-//     particle's anchor node;
+//   * FP32-compensated form only: a 32-byte record per node (Rec32: local position, local
+//     displacement, cnot * volume), double-buffered; local = relative to the particle's anchor node;
 //   * contact broad phase: hashed cell list (counting sort) rebuilt only when the nodes may
 //     have moved more than half the skin since the last build; per-node candidate lists
 //     (fixed capacity, ascending file index) of nodes within contact radius + skin.
@@ -63,14 +62,25 @@ void parallel_items(uint64_t n, F f) {
 }
 
 constexpr int kSlice = 32;
-constexpr int kStageNodes = 512;          // nodes per block of the staged bond kernel
-constexpr uint32_t kStageMaxRecords = 6400;  // 200 KB of 32-byte records per block
+constexpr int kTileNodes = 256;           // nodes per block of the tiled bond kernel
+constexpr uint32_t kTileRecords = 3072;   // most distinct records a tile may read (12-bit indices)
+constexpr uint16_t kTileBroken = 1;       // flag of a broken (or missing) bond in a tile column entry
+constexpr int kFirstTileVariant = 10, kLastTileVariant = 13;  // bond-kernel variants of the tiled kernel
 constexpr uint32_t kNoCol = 0xFFFFFFFFu;
 constexpr uint16_t kCandCells = 0xFFFFu;  // cand_n of a node whose contact partners come from the cell list
 constexpr uint32_t kMaxCandCap = 64;      // largest per-node candidate list
 constexpr uint32_t kColBroken = 0x80000000u;  // FP32 form: broken flag in a column entry
 constexpr uint32_t kColIndex = 0x7FFFFFFFu;   // the partner index in a column entry
 constexpr uint64_t kOrderWindow = 1024;     // nodes per window of the bond-count sort (order_nodes)
+constexpr uint64_t kOrderWindow32 = 256;    // FP32 form, particles above kOrderWindow nodes: one tile's worth
+// FP32 handles of at least this many nodes (1024 tiles, 2.2 times the 456 resident at once) get the
+// tile arrays when they are created and step with the tiled bond kernel by default. Below, the
+// last, partly filled round of tiles costs more than the tiles save (200k nodes in contact: 98 us
+// against 84 us with the gather-ahead kernel 25; 363k: 121 against 145).
+constexpr uint64_t kTileMinNodes = 1ull << 18;
+// From this many nodes on, the tiled kernel leaves the non-bond work to k_extra32 (778k nodes: 197 us
+// either way, 3.98 M: 935 against 961 us fused; 363k in contact: 132 against 121 us).
+constexpr uint64_t kTileSplitNodes = 1ull << 21;
 
 // Per-particle parameters (ParticleN scalars, particle2.h:51-59).
 struct DevPart {
@@ -139,11 +149,17 @@ struct DevCounters {
 };
 
 // FP32 form: one 32-byte record per node, so that a bond gathers its partner with a single
-// 256-bit load: p = (anchor-relative position, cnot * volume), u = (anchor-relative
-// displacement, 0).
+// 256-bit load: the anchor-relative position p and displacement u, and w = cnot * volume. The order
+// lets the tiled bond kernel copy the parts it keeps in shared memory as they lie, x and y of each
+// vector side by side (16 bytes) and both z (8).
 struct __align__(32) Rec32 {
-  float4 p, u;
+  float px, py, ux, uy, pz, uz, w, pad;
 };
+// The displacement part of a record.
+__device__ __forceinline__ void set_rec_u(Rec32 &r, float x, float y, float z) {
+  *reinterpret_cast<float2 *>(&r.ux) = make_float2(x, y);
+  r.uz = z;
+}
 
 // An entry of the broad phase's cell list: the node's position inside its cell (in cell edges),
 // its cell (cell coordinates modulo 2^32) and its simulation. 32 bytes, so that a candidate is
@@ -186,10 +202,16 @@ struct DevView {
   double *anchor_next;        // [P][3] anchor of rec_next[].u
   double break_band;     // relative band around snot where the FP64 stretch decides
   double *f_extra;       // [3][Ncap] FP64 non-bond force density of flagged nodes
-  // FP32 form, staged bond kernel: per block of kStageNodes nodes, the contiguous range of
-  // node records its bonds read ([win_lo, win_lo + win_cnt); win_cnt 0 = not staged)
-  const uint32_t *win_lo, *win_cnt;
-  uint32_t win_max;      // largest staged range (records): the kernel's shared-memory size
+  // FP32 form, tiled bond kernel (prepare_tiles): per tile of kTileNodes nodes, the list of the
+  // distinct records its bonds read ([ntiles][kTileRecords], tile_n of them; 0: more than fit, the
+  // tile gathers from global memory), and per bond the partner's place in that list: 16 bits (place
+  // * 16 + broken flag), four consecutive positions of a row side by side, the 32 rows of a slice
+  // in turn
+  const uint32_t *tile_rec, *tile_n;
+  uint16_t *tcol;
+  uint32_t tile_max;     // longest list: the kernel's shared-memory size in records
+  uint32_t tile_gather;  // tiles whose records do not fit
+  int tile_vol;          // 1: records carry cnot * volume (it varies inside a particle), 0: one per particle
   // FP32 form: work lists of k_extra32 (see BroadPhase)
   uint32_t *xnodes, *xparts, *xcount;
   uint32_t max_part_nodes;  // nodes of the largest particle
@@ -365,6 +387,7 @@ class Engine {
   // from the save would have. A finished simulation cannot be saved (its device state is gone).
   int save_sim(uint32_t sim, std::vector<uint8_t> &out);
   int load_sim(uint32_t sim, const uint8_t *buf, uint64_t n);
+  std::vector<uint32_t> ckpt_order(uint32_t sim) const;
   // Bytes of device memory this engine holds, and the same figure computed from a setup
   // before anything is allocated.
   uint64_t device_bytes() const { return device_bytes_; }
@@ -372,18 +395,19 @@ class Engine {
   // setups pd_create_batch would refuse).
   static uint64_t estimate_bytes(const std::vector<HostSim> &sims, int precision, uint32_t cand_cap,
                                  int64_t *bad = nullptr);
-  // Engine node order: inside each window of kOrderWindow nodes of a particle, nodes by
-  // descending bond count bin (stable: equal bins keep their file order). file_of[engine index] = file index, node_of = its inverse,
+  // Engine node order. FP64 form: inside each window of kOrderWindow nodes of a particle, nodes by
+  // descending bond count (stable: equal counts keep their file order). FP32 form: a particle of
+  // more than kOrderWindow nodes along a Morton curve of cells of ~64 nodes (file order inside a
+  // cell), then inside each window of kOrderWindow32 nodes by descending bond count / 16; smaller
+  // particles as the FP64 form, by count / 16. file_of[engine index] = file index, node_of = its inverse,
   // deg_file = bond count of each node in file order (indices out of range are not counted).
   static void order_nodes(const std::vector<HostSim> &sims, std::vector<uint32_t> &file_of,
                           std::vector<uint32_t> &node_of, std::vector<uint32_t> &deg_file,
                           int64_t *bad = nullptr,   // a particle with an index out of range, or -1
                           bool *sorted = nullptr,   // every Connectivity strictly (i, j)-sorted, i < j
-                          uint32_t deg_bin = 1);    // sort by bond count / deg_bin (order_bin)
-  // Bond-count bin of the node order for a precision form: exact counts for the FP64 form (its
-  // padded SELL lanes idle through FP64 arithmetic), bins of 16 for the FP32 form (its record
-  // gathers keep more of the file's lattice locality, at a few per cent more padding).
-  static uint32_t order_bin(int precision) { return precision == PD_FP32C ? 16u : 1u; }
+                          int precision = PD_FP64);
+  // SELL rows of a slice are padded to this multiple (the tiled bond kernel reads positions in fours).
+  static uint32_t row_pad(int precision) { return precision == PD_FP32C ? 4u : 1u; }
   int raw_alloc(void **p, size_t bytes);
   double step_bytes(uint64_t live_bonds) const;
   uint64_t initial_bonds() const { return initial_bonds_; }
@@ -421,16 +445,20 @@ class Engine {
   // Bond counts per engine node (deg), h_deg_, h_slice_ptr_, E_, initial_bonds_, and the row
   // starts of a row-contiguous layout when rowptr is given.
   int bond_counts(std::vector<uint32_t> &deg, std::vector<uint64_t> *rowptr);
-  int alloc_bond_arrays();  // device SELL arrays (+ staged-kernel ranges), slice_ptr and deg uploaded
+  int alloc_bond_arrays();  // device SELL arrays, slice_ptr and deg uploaded
   // Device build from a sorted Connectivity, after bond_counts (rowptr: its row starts);
   // fallback = true when its scratch does not fit.
   int build_bonds_gpu(const std::vector<uint64_t> &rowptr, bool &fallback);
   int launch_step_seq(int cur, cudaStream_t s);
+  bool tile_variant() const { return variant_ >= kFirstTileVariant && variant_ <= kLastTileVariant; }
   int prepare_fused(int cur);  // FP32 form: predicted state for the next step from disp[cur^1]
   int capture_graphs();
-  // FP32 form: record ranges of the staged bond kernel (win_lo / win_cnt / win_max), computed
-  // on the device the first time a staged variant is needed.
-  int prepare_windows();
+  // FP32 form: the tile arrays of the tiled bond kernel, built on the device the first time they
+  // are needed (at creation from kTileMinNodes nodes on).
+  int prepare_tiles();
+  // Before steps are launched: the tile columns' broken flags follow the masks if other kernels have
+  // stepped since the tiled one last did.
+  int refresh_tiles(bool tiled);
   // One step graph whose broad-phase rebuild kernels sit in a conditional node set by
   // k_bp_decide (0 on success; falls back to the plain graph when unsupported).
   int capture_conditional(int cur, cudaGraphExec_t *out);
@@ -513,9 +541,12 @@ class Engine {
   double *d_bxi_ = nullptr, *d_bxin_ = nullptr, *d_brxin_ = nullptr;
   double *d_anchor_ = nullptr;
   double *d_f_extra_ = nullptr;
-  uint32_t *d_win_lo_ = nullptr, *d_win_cnt_ = nullptr;
-  uint32_t win_max_ = 0;
-  bool windows_ready_ = false;
+  uint32_t *d_tile_rec_ = nullptr, *d_tile_n_ = nullptr;
+  uint16_t *d_tcol_ = nullptr;
+  uint32_t tile_max_ = 0;
+  uint32_t tiles_gathering_ = 0;  // tiles whose records do not fit
+  bool tile_vol_ = false;         // see DevView
+  bool tiles_ready_ = false, tiles_stale_ = false;
   uint8_t *d_extra_flag_ = nullptr;
   float *d_wall_local_ = nullptr;
   unsigned int *d_lrtb_local_ = nullptr;
@@ -590,12 +621,10 @@ void launch_predict(const DevView &v, int tpb, cudaStream_t s);
 void launch_step_kernel(const DevView &v, int precision, int variant, cudaStream_t s);
 void launch_step_fp32c(const DevView &v, int variant, cudaStream_t s);
 int num_bond_variants();
-// Raises the dynamic shared-memory limit of the staged bond kernels (once per engine).
-int prepare_staged_kernels(uint32_t smem_bytes);
-constexpr int kFirstStagedVariant = 10;  // variants >= this use the staged bond kernel
-// Per block of kStageNodes nodes, the smallest contiguous range of node records that holds the
-// block's own nodes and every partner of their bonds (win_cnt 0 when above kStageMaxRecords).
-void launch_stage_windows(const DevView &v, uint32_t *win_lo, uint32_t *win_cnt, cudaStream_t s);
+// Raises the dynamic shared-memory limit of the tiled bond kernels.
+cudaError_t prepare_tile_kernels();
+// Builds the tile arrays (DevView::tile_rec, tile_n, tcol) from the column entries (pd_tile.cu).
+cudaError_t launch_tile_build(const DevView &v, uint32_t *tile_rec, uint32_t *tile_n, uint16_t *tcol, cudaStream_t s);
 void launch_end_step(const DevView &v, const uint32_t *clamped, uint64_t n_clamped, double *clamped_disp,
                      cudaStream_t s);
 void launch_centroids(const DevView &v, cudaStream_t s);

@@ -59,8 +59,8 @@ __device__ __forceinline__ ExtraCtx extra_ctx(const DevView &v, uint64_t n, cons
   c.mov = P.movable != 0;
   c.wall_near = false;
   if (c.mov && P.stoppable && sp.allow_wall) {
-    const float4 pl = v.rec[n].p, ul = v.rec[n].u;
-    const float cx = pl.x + ul.x, cy = pl.y + ul.y, cz = pl.z + ul.z;
+    const Rec32 r = v.rec[n];
+    const float cx = r.px + r.ux, cy = r.py + r.uy, cz = r.pz + r.uz;
     const float *wl = v.wall_local + 6 * (uint64_t)c.k;
     const float lim = (float)sp.Rc * 1.001f;
     c.wall_near = fabsf(cx - wl[0]) <= lim || fabsf(cx - wl[3]) <= lim || fabsf(cy - wl[1]) <= lim ||
@@ -295,7 +295,10 @@ __device__ __forceinline__ void extra_node(const DevView &v, uint64_t n) {
   const uint32_t k = v.pid[n];
   const DevPart &P = v.parts[k];
   const DevSimState &st = v.ss[P.sim];
-  if (!st.active || !extra_needed(v, n, k, P, v.sp[P.sim], st, v.rec[n].p, v.rec[n].u)) return;
+  const Rec32 r = v.rec[n];
+  if (!st.active || !extra_needed(v, n, k, P, v.sp[P.sim], st, make_float4(r.px, r.py, r.pz, r.w),
+                                  make_float4(r.ux, r.uy, r.uz, 0.f)))
+    return;
   st3(v.f_extra, n, v.Ncap, extra_force(v, n));
   v.extra_flag[n] = 1;
 }
@@ -307,8 +310,25 @@ __global__ void __launch_bounds__(128) k_extra32(const __grid_constant__ DevView
     return;
   }
   const uint32_t nx = v.xcount[0], np = v.xcount[1];
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nx; i += gridDim.x * blockDim.x)
-    extra_node(v, v.xnodes[i]);
+  // Nodes with contact candidates: four lanes each, sharing the listed candidates (a pair in contact
+  // is a chain of FP64 square roots and divisions, ~2 us; with one thread per node the kernel waited
+  // for the longest list).
+  const uint32_t sub = threadIdx.x & 3u, first = (threadIdx.x & 31u) - sub;
+  for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 2; i < nx; i += (gridDim.x * blockDim.x) >> 2) {
+    const uint64_t n = v.xnodes[i];
+    const uint32_t sim = v.parts[v.pid[n]].sim;
+    if (!v.ss[sim].active) continue;  // the group's four lanes together
+    D3 f;
+    if (v.cand_n[n] == kCandCells) {  // the cell walk: one lane
+      if (sub == 0) f = extra_force(v, n);
+    } else {
+      f = extra_force_lanes<4>(v, n, sub, first);
+    }
+    if (sub == 0) {
+      st3(v.f_extra, n, v.Ncap, f);
+      v.extra_flag[n] = 1;
+    }
+  }
   // the listed particles' nodes in chunks of one block's threads, spread over all blocks (one
   // block per particle left a 10k-node particle's nodes to 128 threads in turn)
   const uint64_t cpp = (v.max_part_nodes + blockDim.x - 1) / blockDim.x;  // chunks per particle
@@ -359,27 +379,27 @@ __device__ __forceinline__ uint32_t ld_col(const uint32_t *p) {
   return r;
 }
 
-// A partner's record: one 256-bit load (W) or two 128-bit loads of the same 32-byte sector;
-// NC = 0 as for ld_col.
+// A partner's record as p = (position, cnot * volume) and u = (displacement, 0): one 256-bit load
+// (W) or two 128-bit loads of the same 32-byte sector; NC = 0 as for ld_col.
 template <int W, int NC = 1>
 __device__ __forceinline__ void ld_rec(const Rec32 *r, float4 &p, float4 &u) {
   if (W && NC) {
     asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-        : "=f"(p.x), "=f"(p.y), "=f"(p.z), "=f"(p.w), "=f"(u.x), "=f"(u.y), "=f"(u.z), "=f"(u.w)
+        : "=f"(p.x), "=f"(p.y), "=f"(u.x), "=f"(u.y), "=f"(p.z), "=f"(u.z), "=f"(p.w), "=f"(u.w)
         : "l"(r));
   } else if (W) {
     asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=f"(p.x), "=f"(p.y), "=f"(p.z), "=f"(p.w), "=f"(u.x), "=f"(u.y), "=f"(u.z), "=f"(u.w)
+                 : "=f"(p.x), "=f"(p.y), "=f"(u.x), "=f"(u.y), "=f"(p.z), "=f"(u.z), "=f"(p.w), "=f"(u.w)
                  : "l"(r)
                  : "memory");
   } else if (NC) {
-    p = __ldg(&r->p);
-    u = __ldg(&r->u);
+    asm("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(p.x), "=f"(p.y), "=f"(u.x), "=f"(u.y) : "l"(&r->px));
+    asm("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(p.z), "=f"(u.z), "=f"(p.w), "=f"(u.w) : "l"(&r->pz));
   } else {
     asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
-                 : "=f"(p.x), "=f"(p.y), "=f"(p.z), "=f"(p.w) : "l"(&r->p) : "memory");
+                 : "=f"(p.x), "=f"(p.y), "=f"(u.x), "=f"(u.y) : "l"(&r->px) : "memory");
     asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
-                 : "=f"(u.x), "=f"(u.y), "=f"(u.z), "=f"(u.w) : "l"(&r->u) : "memory");
+                 : "=f"(p.z), "=f"(u.z), "=f"(p.w), "=f"(u.w) : "l"(&r->pz) : "memory");
   }
 }
 
@@ -460,6 +480,9 @@ __device__ __forceinline__ void kahan_merge(Acc32 &a, const Acc32 &b) {
   merge1(a.sz, a.cz, b.sz, b.cz);
 }
 __device__ __forceinline__ D3 acc_value(const Acc32 &a) {
+  if (!(odd_float(a.sx) || odd_float(a.sy) || odd_float(a.sz) || odd_float(a.cx) || odd_float(a.cy) ||
+        odd_float(a.cz)))
+    return d3(widen(a.sx) - widen(a.cx), widen(a.sy) - widen(a.cy), widen(a.sz) - widen(a.cz));
   return d3((double)a.sx - (double)a.cx, (double)a.sy - (double)a.cy, (double)a.sz - (double)a.cz);
 }
 // Lane src's accumulator, all lanes taking part.
@@ -554,70 +577,78 @@ __device__ __forceinline__ void verlet_tail(const DevView &v, uint64_t nn, uint3
   const int32_t movable = P.movable;
   float i2 = 0.f;  // squared displacement increment of the next step (broad-phase bound)
   if (run) {
-    st3(v.force, nn, C3, f);
-    if (nonfinite(f.x) || nonfinite(f.y) || nonfinite(f.z)) atomicOr(&v.cnt->err, PD_DERR_NONFINITE);
-    const D3 vi = ld3(v.vel_in, nn, C3);
-    D3 vo = vi;
-    D3 an = ld3(v.acc, nn, C3);
+    // every load before the first store: the compiler cannot move a load above a store that might
+    // alias it, and each load left behind one costs its whole latency
     const DevSimParams &sp = v.sp[P.sim];
+    const D3 vi = ld3(v.vel_in, nn, C3), ao = ld3(v.acc, nn, C3), d = ld3(v.disp, nn, C3);
+    const double *anx = v.anchor_next + 3 * (uint64_t)k;
+    const D3 anchor = d3(anx[0], anx[1], anx[2]);
     const bool clamped = movable && v.clamp_flag[nn];
-    if (movable) {
-      // velocity-Verlet corrector (timeloop.h:670-682)
-      const D3 ao = an;
-      if (v.afd && st.vconstraint && (int32_t)(k - sp.p0) == sp.pv_particle) st3(v.afd, nn, C3, ao);
+    D3 vo = vi, an = ao;
+    if (movable) {  // velocity-Verlet corrector (timeloop.h:670-682)
       an = P.irho * f;
       vo = vi + sp.hdt * (ao + an);
-      if (clamped) {  // timeloop.h:767-774
-        vo = d3(0.0, 0.0, 0.0);
-        an = d3(0.0, 0.0, 0.0);
-      }
+    }
+    if (clamped) {  // timeloop.h:767-774
+      vo = d3(0.0, 0.0, 0.0);
+      an = d3(0.0, 0.0, 0.0);
+    }
+    // predictor of the next step (timeloop.h:537-540)
+    D3 dn, inc;
+    if (clamped) {
+      dn = d3(0.0, 0.0, 0.0);
+      inc = d;  // its length counts
+    } else {
+      inc = sp.dt * vo + sp.hdt2 * an;
+      dn = d + inc;
+    }
+    st3(v.force, nn, C3, f);
+    if (nonfinite(f.x) || nonfinite(f.y) || nonfinite(f.z)) atomicOr(&v.cnt->err, PD_DERR_NONFINITE);
+    if (movable) {
+      if (v.afd && st.vconstraint && (int32_t)(k - sp.p0) == sp.pv_particle) st3(v.afd, nn, C3, ao);
       st3(v.acc, nn, C3, an);
     }
     st3(v.vel_out, nn, C3, vo);
-    // predictor of the next step (timeloop.h:537-540)
-    const D3 d = ld3(v.disp, nn, C3);
-    D3 dn;
-    if (clamped) {
-      dn = d3(0.0, 0.0, 0.0);
-    } else {
-      const D3 inc = sp.dt * vo + sp.hdt2 * an;
-      dn = d + inc;
-    }
     st3(v.disp_next, nn, C3, dn);
-    const float ix = (float)(dn.x - d.x), iy = (float)(dn.y - d.y), iz = (float)(dn.z - d.z);
+    set_rec_u(v.rec_next[nn], narrow(dn.x - anchor.x), narrow(dn.y - anchor.y), narrow(dn.z - anchor.z));
+    const float ix = magnitude(inc.x), iy = magnitude(inc.y), iz = magnitude(inc.z);
     i2 = ix * ix + iy * iy + iz * iz;
-    const double *anx = v.anchor_next + 3 * (uint64_t)k;
-    v.rec_next[nn].u = make_float4((float)(dn.x - anx[0]), (float)(dn.y - anx[1]), (float)(dn.z - anx[2]), 0.f);
   }
-  // particle AABB of this step's positions in the particle's local frame
+  // particle AABB of this step's positions in the particle's local frame, reduced over the warp as
+  // ordered keys (one instruction each; a NaN coordinate counts as absent)
   {
     const bool contrib = run && movable;
-    const float px = pi4.x + ui4.x, py = pi4.y + ui4.y, pz = pi4.z + ui4.z;
-    float lo[3] = {contrib ? px : INFINITY, contrib ? py : INFINITY, contrib ? pz : INFINITY};
-    float hi[3] = {contrib ? px : -INFINITY, contrib ? py : -INFINITY, contrib ? pz : -INFINITY};
+    const float x[3] = {pi4.x + ui4.x, pi4.y + ui4.y, pi4.z + ui4.z};
+    unsigned int lo[3], hi[3];
+    for (int c = 0; c < 3; ++c) {
+      const bool on = contrib && x[c] == x[c];
+      lo[c] = on ? fkey(x[c]) : fkey(INFINITY);
+      hi[c] = on ? fkey(x[c]) : fkey(-INFINITY);
+    }
     const uint32_t k0 = __shfl_sync(0xffffffffu, k, 0);
     const bool uniform = __all_sync(0xffffffffu, k == k0);
     if (uniform) {
-      for (int o = 16; o > 0; o >>= 1) {
-        for (int c = 0; c < 3; ++c) {
-          lo[c] = fminf(lo[c], __shfl_xor_sync(0xffffffffu, lo[c], o));
-          hi[c] = fmaxf(hi[c], __shfl_xor_sync(0xffffffffu, hi[c], o));
-        }
+      for (int c = 0; c < 3; ++c) {
+        lo[c] = __reduce_min_sync(0xffffffffu, lo[c]);
+        hi[c] = __reduce_max_sync(0xffffffffu, hi[c]);
       }
     }
     const bool writer = uniform ? ((threadIdx.x & 31) == 0) : contrib;
     if (writer && lo[0] <= hi[0]) {
       unsigned int *L = v.lrtb_local_next + 6 * (uint64_t)k;
       for (int c = 0; c < 3; ++c) {
-        atomicMin(&L[c], fkey(lo[c]));
-        atomicMax(&L[3 + c], fkey(hi[c]));
+        atomicMin(&L[c], lo[c]);
+        atomicMax(&L[3 + c], hi[c]);
       }
     }
   }
-  for (int o = 16; o > 0; o >>= 1) i2 = fmaxf(i2, __shfl_xor_sync(0xffffffffu, i2, o));
+  // the warp's largest increment: an upper bound (the factor covers the truncated magnitudes and the
+  // FP32 roundings), taken in FP32 -- the square root of one lane in FP64 was a quarter of the
+  // corrector's FP64 work
+  i2 = __uint_as_float(__reduce_max_sync(0xffffffffu, i2 > 0.f ? __float_as_uint(i2) : 0u));
   if ((threadIdx.x & 31) == 0 && i2 > 0.f) {
-    const double inc = sqrt((double)i2) * (1.0 + 1e-5);
-    atomicMax(&v.cnt->stepmax_bits, (unsigned long long)__double_as_longlong(inc));
+    const float inc = __fmul_ru(__fsqrt_ru(i2), 1.00001f);
+    atomicMax(&v.cnt->stepmax_bits, (unsigned long long)__double_as_longlong(odd_float(inc) ? (double)inc : widen(inc)));
   }
 }
 
@@ -943,160 +974,289 @@ __global__ void __launch_bounds__(128, MINB) k_bond32(const __grid_constant__ De
   bond_node<U, W, PF, FX>(v, (uint64_t)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
-// Staged form of the bond kernel: one block of kStageNodes nodes first copies the contiguous
-// range of node records its bonds read into shared memory with bulk asynchronous copies
-// (cp.async.bulk, completion on an mbarrier), then gathers every partner from shared memory
-// instead of L1/L2. Blocks whose range does not fit (win_cnt == 0), or whose copy misses the
-// wait limit, read global memory as the plain kernel does; results are the same either way.
-constexpr uint32_t kStageWaitPolls = 1u << 22;  // bounded wait (~0.5 s) for the staging copy
+// ---- the tiled bond kernel (large handles) -------------------------------------------------
+//
+// One block per tile of kTileNodes consecutive nodes. The engine order keeps a tile's nodes
+// together in space, so its ~24,000 bonds read only ~1,450 distinct partner records: the block
+// copies those into shared memory once and gathers every partner from there, by the 16-bit places
+// of the tile's own column stream (half the bytes of the 32-bit one).
+// What bounds it: the load/store data pipe (shared memory's wavefronts) with the issue slots and the
+// FP64 corrector close behind. Gathering records through L1 cost 22 wavefronts per position of a
+// warp (32 bonds), the pipe 81 % busy; from shared memory a partner is one 16-byte and one 8-byte
+// load, ~14 wavefronts (random bank conflicts; 6 at best). The record is split for that: (px, py, ux,
+// uy) and (pz, uz); cnot * volume, the same for all nodes of a particle on a lattice of equal
+// volumes, then comes from the node's own record (VOL = 1: it is read with the partner, two 16-byte
+// loads). The stretch and the Kahan sums take x and y in one packed FP32 instruction (f32x2: the same
+// roundings per half), z apart. Three blocks per SM: a block's copy and its corrector are latency
+// (11 us of a tile's 30), which the other blocks' loops overlap.
+// Measured (bond phase per step, 3.98 M / 778k / 363k nodes): 1180 / 244 / 156 us gathering through
+// L1 (variant 18), 1130 / 232 / 147 us with the shorter corrector, tiled 935 / 197 / 121 us.
+// Every expression and the order of the sums are bond_node's, so the results are the same bits.
 
-template <int U, int PF>
-__global__ void __launch_bounds__(kStageNodes, 1) k_bond32s(const __grid_constant__ DevView v) {
-  extern __shared__ __align__(128) unsigned char stage_raw[];
-  Rec32 *win = reinterpret_cast<Rec32 *>(stage_raw);
-  __shared__ __align__(8) uint64_t bar;
+// Place of position j of a row (its lane in the slice at sbase) in the tile column stream.
+__host__ __device__ __forceinline__ uint64_t tile_entry(uint64_t sbase, uint32_t j, uint32_t lane) {
+  return sbase + 128ull * (j >> 2) + 4ull * lane + (j & 3u);
+}
+// Shared bytes per record.
+__host__ __device__ constexpr uint32_t tile_rec_bytes(int vol) { return vol ? 32u : 24u; }
+
+typedef unsigned long long f32x2;  // two floats (low, high) in a 64-bit register
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 a) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
+  return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+// Acc32 with x and y packed and the compensations negated (nc = -c), so that every difference of
+// the sum is one packed multiply-add: a - b as b * (-1) + a, rounded once.
+struct AccT {
+  f32x2 s, nc;
+  float sz, ncz;
+};
+__device__ __forceinline__ Acc32 acc32(const AccT &a) {
+  const float2 s = unpack2(a.s), c = unpack2(a.nc);
+  return Acc32{s.x, s.y, a.sz, -c.x, -c.y, -a.ncz};
+}
+
+// bond32_terms with x and y packed.
+struct BondT {
+  f32x2 y;
+  float yz, g, str;
+};
+struct OwnT {  // the node's own coordinates, negated
+  f32x2 np, nu, nz;
+};
+__device__ __forceinline__ BondT tile_terms(const OwnT &o, f32x2 p, f32x2 u, f32x2 z, float w) {
+  BondT b;
+  const f32x2 xi = add2(p, o.np), eta = add2(u, o.nu), xe = add2(z, o.nz);
+  b.y = add2(xi, eta);
+  const float2 x = unpack2(xi), e = unpack2(eta), y = unpack2(b.y), ze = unpack2(xe), xy = unpack2(add2(xi, b.y));
+  b.yz = ze.x + ze.y;
+  const float x2 = fmaf(x.x, x.x, fmaf(x.y, x.y, ze.x * ze.x));
+  const float y2 = fmaf(y.x, y.x, fmaf(y.y, y.y, b.yz * b.yz));
+  const float num = fmaf(e.x, xy.x, fmaf(e.y, xy.y, ze.y * (ze.x + b.yz)));
+  const float rx = rsqrt_approx(x2), ry = rsqrt_approx(y2);
+  b.str = (num * rx) * rcp_approx(fmaf(x2, rx, y2 * ry));
+  b.g = (b.str * ry) * w;
+  return b;
+}
+__device__ __forceinline__ void tile_add(AccT &a, const BondT &b) {
+  const f32x2 m1 = pack2(-1.0f, -1.0f);
+  const f32x2 y = fma2(pack2(b.g, b.g), b.y, a.nc), t = add2(a.s, y);
+  a.nc = fma2(fma2(a.s, m1, t), m1, y);
+  a.s = t;
+  const float yz = fmaf(b.g, b.yz, a.ncz), tz = a.sz + yz;
+  a.ncz = yz - (tz - a.sz);
+  a.sz = tz;
+}
+
+// The tiles whose records do not fit in shared memory (launched where there are any).
+template <int FX>
+__global__ void __launch_bounds__(kTileNodes, 2) k_bond32g(const __grid_constant__ DevView v) {
+  if (v.tile_n[blockIdx.x] == 0) bond_node<4, 1, 1, FX>(v, (uint64_t)blockIdx.x * kTileNodes + threadIdx.x);
+}
+
+// BYTES from global to shared memory without passing through registers.
+template <int BYTES>
+__device__ __forceinline__ void copy_async(uint32_t dst, const void *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst), "l"(src), "n"(BYTES) : "memory");
+}
+
+// Brings this thread's line of a node array into L2 ahead of the corrector's loads.
+__device__ __forceinline__ void prefetch3(const double *a, uint64_t n, uint64_t cap) {
+  for (int c = 0; c < 3; ++c) asm volatile("prefetch.global.L2 [%0];" ::"l"(a + n + c * cap));
+}
+
+// A bond's terms from its tile column entry (at: its place * 16). A, B: shared addresses of the two
+// record parts.
+template <int VOL>
+__device__ __forceinline__ BondT tile_bond(uint32_t at, uint32_t A, uint32_t B, const OwnT &own, float w) {
+  f32x2 p, d, z, wz;
+  asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(p), "=l"(d) : "r"(A + at));
+  if (VOL) {
+    asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(z), "=l"(wz) : "r"(B + at));
+    return tile_terms(own, p, d, z, unpack2(wz).x);
+  }
+  asm volatile("ld.shared.b64 %0, [%1];" : "=l"(z) : "r"(B + (at >> 1)));
+  return tile_terms(own, p, d, z, w);
+}
+
+// One group of four positions of a row, U of them in flight together; LIVE: all four bonds are.
+// Returns the largest live stretch.
+template <int U, int VOL, bool LIVE>
+__device__ __forceinline__ float tile_group(const uint2 c, uint32_t A, uint32_t B, const OwnT &own, float w, AccT &a) {
+  float top = -INFINITY;
+  const uint32_t r[4] = {c.x & 0xFFFFu, c.x >> 16, c.y & 0xFFFFu, c.y >> 16};
+#pragma unroll
+  for (int h = 0; h < 4; h += U) {
+    BondT b[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) b[u] = tile_bond<VOL>(LIVE ? r[h + u] : r[h + u] & 0xFFF0u, A, B, own, w);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (LIVE || !(r[h + u] & kTileBroken)) {
+        tile_add(a, b[u]);
+        top = fmaxf(top, b[u].str);
+      }
+  }
+  return top;
+}
+
+__device__ __forceinline__ OwnT tile_own(const float4 &p, const float4 &u) {
+  return OwnT{pack2(-p.x, -p.y), pack2(-u.x, -u.y), pack2(-p.z, -u.z)};
+}
+
+// The breaking decisions of a row, in the groups where some live stretch reaches the band around
+// snot (bit g mod 32 of groups): a second evaluation of those groups out of the bond loop, which
+// keeps the loop free of the decisions' registers and branches. A bond breaks when its FP32 stretch
+// is past the band, else as FP64 decides (band_check); its column entries follow.
+template <int VOL>
+__device__ __noinline__ void tile_break_row(const DevView &v, uint64_t n, uint32_t A, uint32_t B, uint32_t groups) {
+  const uint32_t lane = (uint32_t)(n & 31);
+  const uint64_t sbase = v.slice_ptr[n >> 5];
+  const DevPart &P = v.parts[v.pid[n]];
+  float4 p, u;
+  ld_rec<0>(v.rec + n, p, u);
+  const OwnT own = tile_own(p, u);
+  const int dg = v.deg[n];
+  const float slo = P.snot_lo32, shi = P.snot_hi32;
+  for (int g = 0; 4 * g < dg; ++g) {
+    if (!((groups >> (g & 31)) & 1u)) continue;
+    uint16_t *tc = v.tcol + tile_entry(sbase, 4u * g, lane);
+    const uint2 c = *reinterpret_cast<const uint2 *>(tc);
+    const uint32_t r[4] = {c.x & 0xFFFFu, c.x >> 16, c.y & 0xFFFFu, c.y >> 16};
+    float s[4];
+#pragma unroll
+    for (int h = 0; h < 4; ++h) s[h] = tile_bond<VOL>(r[h] & 0xFFF0u, A, B, own, p.w).str;
+    for (int h = 0; h < 4; ++h) {
+      if ((r[h] & kTileBroken) || !(s[h] > slo)) continue;
+      const int j = 4 * g + h;
+      uint32_t *word = v.mask + (sbase >> 5) + j;
+      uint32_t *cole = const_cast<uint32_t *>(v.col) + sbase + lane + 32ull * j;
+      const uint32_t q = *cole & kColIndex;
+      if (s[h] > shi) cut_bond(word, lane, cole, q);
+      else band_check(v, n, q, word, lane, P.snot, cole);
+      if (*(volatile uint32_t *)cole & kColBroken) tc[h] |= kTileBroken;
+    }
+  }
+}
+
+// MINB: blocks per SM (register cap); U: positions whose loads and terms are in flight together; FX:
+// the FP64 non-bond work is done here instead of in k_extra32.
+template <int MINB, int U, int VOL, int FX>
+__global__ void __launch_bounds__(kTileNodes, MINB) k_bond32t(const __grid_constant__ DevView v) {
+  extern __shared__ __align__(16) unsigned char tile_smem[];
+  __shared__ float tot_sh[6][kTileNodes];  // merged blocks of each row so far: used four times, kept out of registers
   if (blockIdx.x == 0 && threadIdx.x == 0 && v.xcount) {  // as in k_bond32
     v.xcount[1] = 0;
     v.cnt->xall = 0;
   }
-  const uint32_t wlo = v.win_lo[blockIdx.x];
-  const uint32_t wcnt = v.win_cnt[blockIdx.x];
-  bool staged = wcnt != 0;
-  bool copy_done = true;
-  if (staged) {
-    if (threadIdx.x == 0) {
-      mbar_init(&bar, 1);
-      const uint32_t bytes = wcnt * (uint32_t)sizeof(Rec32);
-      mbar_expect_tx(&bar, bytes);
-      const char *src = reinterpret_cast<const char *>(v.rec + wlo);
-      for (uint32_t off = 0; off < bytes; off += 32768u)
-        bulk_g2s(stage_raw + off, src + off, bytes - off < 32768u ? bytes - off : 32768u, &bar);
-    }
-    __syncthreads();  // the barrier is initialised before anyone polls it
-    copy_done = mbar_wait_bounded(&bar, 0, kStageWaitPolls);
-    staged = __syncthreads_and(copy_done) != 0;
-    if (!staged && threadIdx.x == 0) atomicOr(&v.cnt->err, PD_DERR_STAGE_TIMEOUT);
-  }
-  const uint64_t n = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t A = (uint32_t)__cvta_generic_to_shared(tile_smem), B = A + 16 * v.tile_max;
+  const uint64_t n = (uint64_t)blockIdx.x * kTileNodes + threadIdx.x;
   const bool valid = n < v.N;
   const uint64_t nn = valid ? n : 0;
+  {
+    constexpr int kAhead = 6;  // list entries requested together with the list's length
+    const uint32_t *list = v.tile_rec + (uint64_t)blockIdx.x * kTileRecords + threadIdx.x;
+    uint32_t q[kAhead];
+#pragma unroll
+    for (int i = 0; i < kAhead; ++i) q[i] = list[i * kTileNodes];
+    const uint32_t cnt = v.tile_n[blockIdx.x];
+    if (cnt == 0) return;  // k_bond32g's
+    const Rec32 *rec = v.rec;
+    auto copy = [&](uint32_t i, uint32_t from) {
+      const Rec32 *r = rec + from;
+      copy_async<16>(A + 16 * i, &r->px);
+      if (VOL) copy_async<16>(B + 16 * i, &r->pz);
+      else copy_async<8>(B + 8 * i, &r->pz);
+    };
+#pragma unroll
+    for (int i = 0; i < kAhead; ++i)
+      if (threadIdx.x + i * kTileNodes < cnt) copy(threadIdx.x + i * kTileNodes, q[i]);
+    for (uint32_t i = kAhead * kTileNodes; threadIdx.x + i < cnt; i += kTileNodes) copy(threadIdx.x + i, list[i]);
+  }
   const uint32_t k = v.pid[nn];
   const DevPart &P = v.parts[k];
-  const int32_t movable = P.movable;
   const DevSimState &st = v.ss[P.sim];
   const bool run = valid && st.active;
-  const uint64_t C3 = v.Ncap;
+  if ((threadIdx.x & 15) == 0 && run) {
+    prefetch3(v.vel_in, nn, v.Ncap);
+    prefetch3(v.acc, nn, v.Ncap);
+    prefetch3(v.disp, nn, v.Ncap);
+  }
+  const bool work = run && P.movable;
+  if (v.stats) {
+    uint32_t live = work ? row_live(v.col + v.slice_ptr[nn >> 5] + (uint32_t)(nn & 31), v.deg[nn]) : 0u;
+    for (int o = 16; o > 0; o >>= 1) live += __shfl_xor_sync(0xffffffffu, live, o);
+    if ((threadIdx.x & 31) == 0 && live) atomicAdd(&v.cnt->live_bonds, (unsigned long long)live);
+  }
   float4 pi4, ui4;
   ld_rec<1>(v.rec + nn, pi4, ui4);
-  Acc32 tot = {}, a = {};  // merged blocks so far, current block (bond_node)
-  static_assert(U == 4 || U == 8, "groups inside one block of the row");
-  uint32_t live = 0;
-  if (run && movable) {
-    const uint32_t lane = (uint32_t)(nn & 31);
-    const uint64_t sbase = v.slice_ptr[nn >> 5];
-    const uint32_t *colp = v.col + sbase + lane;
-    uint32_t *colw = const_cast<uint32_t *>(colp);
-    uint32_t *maskp = v.mask + (sbase >> 5);
-    const int dg = v.deg[nn];
-    const bool brk = st.fracture && P.breakable && P.break_bonds;
-    const float slo = P.snot_lo32, shi = P.snot_hi32;
-    const Rec32 *__restrict__ rec = v.rec;
-    if (v.stats) live = row_live(colp, dg);
-    // partner record: shared memory when staged (and inside the staged range), else global
-    auto partner = [&](uint32_t q, float4 &p, float4 &u) {
-      const uint32_t o = q - wlo;
-      if (staged && o < wcnt) {
-        p = win[o].p;
-        u = win[o].u;
-      } else {
-        ld_rec<1>(rec + q, p, u);
+  {
+    const int dg = work ? (int)v.deg[nn] : 0, ng = (dg + 3) >> 2;
+    const int cg = chain_len(dg) >> 2;  // a block of the row, in groups of four
+    const uint2 *tc = reinterpret_cast<const uint2 *>(v.tcol + v.slice_ptr[nn >> 5]) + (uint32_t)(nn & 31);
+    const OwnT own = tile_own(pi4, ui4);
+    uint2 c = ng ? __ldg(tc) : make_uint2(0, 0);
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
+    const float slo = st.fracture && P.breakable && P.break_bonds ? P.snot_lo32 : INFINITY;
+    uint32_t near = 0, bit = 1;  // groups with a live stretch in the band around snot or past it
+    int g = 0;
+    for (int m = 0; m < 4; ++m) {  // the row's four blocks (the last ones possibly empty)
+      AccT a = {};
+      const int e = min(ng, cg * (m + 1));
+      for (; g < e; ++g) {
+        const uint2 cn = g + 1 < ng ? __ldg(tc + 32 * (g + 1)) : c;
+        const float top = ((c.x | c.y) & 0x00010001u) == 0 ? tile_group<U, VOL, true>(c, A, B, own, pi4.w, a)
+                                                           : tile_group<U, VOL, false>(c, A, B, own, pi4.w, a);
+        if (top > slo) near |= bit;
+        bit = __funnelshift_l(bit, bit, 1);
+        c = cn;
       }
-    };
-    const int cl = chain_len(dg);
-    int next = cl, merged = 0;
-    int j = 0;
-    uint32_t qb[PF][U];
-#pragma unroll
-    for (int d = 0; d < PF; ++d) {
-      if ((d + 1) * U <= dg) {
-#pragma unroll
-        for (int u = 0; u < U; ++u) qb[d][u] = __ldg(colp + 32 * (d * U + u));
-      }
+      volatile float(*ts)[kTileNodes] = tot_sh;
+      Acc32 tot = {};
+      if (m)
+        tot = Acc32{ts[0][threadIdx.x], ts[1][threadIdx.x], ts[2][threadIdx.x],
+                    ts[3][threadIdx.x], ts[4][threadIdx.x], ts[5][threadIdx.x]};
+      kahan_merge(tot, acc32(a));
+      ts[0][threadIdx.x] = tot.sx;
+      ts[1][threadIdx.x] = tot.sy;
+      ts[2][threadIdx.x] = tot.sz;
+      ts[3][threadIdx.x] = tot.cx;
+      ts[4][threadIdx.x] = tot.cy;
+      ts[5][threadIdx.x] = tot.cz;
     }
-    for (; j + U <= dg; j += U) {
-      uint32_t q[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u) q[u] = qb[0][u];
-#pragma unroll
-      for (int d = 0; d + 1 < PF; ++d) {
-#pragma unroll
-        for (int u = 0; u < U; ++u) qb[d][u] = qb[d + 1][u];
-      }
-      if (j + (PF + 1) * U <= dg) {
-#pragma unroll
-        for (int u = 0; u < U; ++u) qb[PF - 1][u] = __ldg(colp + 32 * (j + PF * U + u));
-      }
-      if (j == next) {  // a new block of the row
-        kahan_merge(tot, a);
-        a = Acc32{};
-        next += cl;
-        ++merged;
-      }
-      float4 pq[U], uq[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u) partner(q[u] & kColIndex, pq[u], uq[u]);
-      BondTerms bt[U];  // as in bond_node: terms unconditionally, live ones summed in order
-#pragma unroll
-      for (int u = 0; u < U; ++u) bt[u] = bond32_terms(pi4, ui4, pq[u], uq[u]);
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        if (!(q[u] & kColBroken)) {
-          kahan_add(a, bt[u].g, bt[u].yx, bt[u].yy, bt[u].yz);
-          if (brk && bt[u].str > slo) {
-            if (bt[u].str > shi) cut_bond(&maskp[j + u], lane, colw + 32 * (j + u), q[u]);
-            else band_check(v, nn, q[u], &maskp[j + u], lane, P.snot, colw + 32 * (j + u));
-          }
-        }
-      }
-    }
-    for (; j < dg; ++j) {
-      if (j == next) {
-        kahan_merge(tot, a);
-        a = Acc32{};
-        next += cl;
-        ++merged;
-      }
-      const uint32_t q = __ldg(colp + 32 * j);
-      if (q & kColBroken) continue;
-      float4 pq, uq;
-      partner(q, pq, uq);
-      const BondTerms b = bond32_terms(pi4, ui4, pq, uq);
-      kahan_add(a, b.g, b.yx, b.yy, b.yz);
-      const float str = b.str;
-      if (brk && str > slo) {
-        if (str > shi) cut_bond(&maskp[j], lane, colw + 32 * j, q);
-        else band_check(v, nn, q, &maskp[j], lane, P.snot, colw + 32 * j);
-      }
-    }
-    kahan_merge(tot, a);  // the last block, then the empty ones: four merges in every form
-    for (++merged; merged < 4; ++merged) kahan_merge(tot, Acc32{});
+    if (near) tile_break_row<VOL>(v, nn, A, B, near);
   }
   D3 f = d3(0.0, 0.0, 0.0);
   if (run) {
-    f = acc_value(tot);
-    if (v.extra_flag[nn]) {
-      f = f + ld3(v.f_extra, nn, C3);
+    const bool extra = FX ? extra_needed(v, nn, k, P, v.sp[P.sim], st, pi4, ui4) : v.extra_flag[nn] != 0;
+    f = acc_value(Acc32{tot_sh[0][threadIdx.x], tot_sh[1][threadIdx.x], tot_sh[2][threadIdx.x],
+                        tot_sh[3][threadIdx.x], tot_sh[4][threadIdx.x], tot_sh[5][threadIdx.x]});
+    if (extra && FX) {
+      f = f + extra_force(v, nn);
+    } else if (extra) {
+      f = f + ld3(v.f_extra, nn, v.Ncap);
       v.extra_flag[nn] = 0;
     }
   }
   verlet_tail(v, nn, k, P, st, run, f, pi4, ui4);
-  if (v.stats) {
-    for (int o = 16; o > 0; o >>= 1) live += __shfl_xor_sync(0xffffffffu, live, o);
-    if ((threadIdx.x & 31) == 0 && live) atomicAdd(&v.cnt->live_bonds, (unsigned long long)live);
-  }
-  // a copy that missed its wait limit may still be writing shared memory: let it land
-  if (!copy_done && threadIdx.x == 0) (void)mbar_wait_bounded(&bar, 0, kStageWaitPolls);
-  __syncthreads();
 }
 
 // ---- the persistent step (small handles) ------------------------------------------------
@@ -1356,54 +1516,22 @@ cudaError_t launch_persist(const PersistArgs &a, uint32_t grid, int lanes, cudaS
   return cudaLaunchCooperativeKernel(persist_kernel(lanes), dim3(grid), dim3(kPersistThreads), args, 0, s);
 }
 
-int prepare_staged_kernels(uint32_t smem_bytes) {
+cudaError_t prepare_tile_kernels() {
+  // the same limits for every handle: the attribute belongs to the kernel, not to a launch
   cudaError_t e = cudaSuccess;
-  auto set = [&](const void *fn) {
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
+  auto set = [&](const void *fn, int vol) {
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kTileRecords * tile_rec_bytes(vol)));
   };
-  set((const void *)k_bond32s<4, 1>);
-  set((const void *)k_bond32s<4, 2>);
-  set((const void *)k_bond32s<4, 3>);
-  set((const void *)k_bond32s<8, 1>);
-  return e == cudaSuccess ? PD_OK : PD_ECUDA;
-}
-
-
-__global__ void k_stage_windows(const __grid_constant__ DevView v, uint32_t *win_lo, uint32_t *win_cnt) {
-  const uint64_t b = blockIdx.x;
-  const uint64_t n0 = b * kStageNodes, n1 = min(v.N, n0 + kStageNodes);
-  uint32_t lo = (uint32_t)n0, hi = (uint32_t)(n1 - 1);
-  const uint64_t e0 = v.slice_ptr[n0 / 32], e1 = v.slice_ptr[(n1 + 31) / 32];
-  for (uint64_t e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
-    const uint32_t q = v.col[e];
-    if (q != kNoCol) {  // a bond, live or broken
-      lo = min(lo, q & kColIndex);
-      hi = max(hi, q & kColIndex);
-    }
-  }
-  lo = __reduce_min_sync(0xffffffffu, lo);
-  hi = __reduce_max_sync(0xffffffffu, hi);
-  __shared__ uint32_t slo[32], shi[32];
-  const int w = threadIdx.x >> 5;
-  if ((threadIdx.x & 31) == 0) {
-    slo[w] = lo;
-    shi[w] = hi;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int i = 1; i < (int)(blockDim.x >> 5); ++i) {
-      lo = min(lo, slo[i]);
-      hi = max(hi, shi[i]);
-    }
-    const uint64_t cnt = (uint64_t)hi - lo + 1;
-    win_lo[b] = lo;
-    win_cnt[b] = cnt <= kStageMaxRecords ? (uint32_t)cnt : 0u;
-  }
-}
-
-void launch_stage_windows(const DevView &v, uint32_t *win_lo, uint32_t *win_cnt, cudaStream_t s) {
-  const uint64_t nb = (v.N + kStageNodes - 1) / kStageNodes;
-  if (nb) k_stage_windows<<<(unsigned)nb, 256, 0, s>>>(v, win_lo, win_cnt);
+  set((const void *)k_bond32t<3, 4, 0, 0>, 0);
+  set((const void *)k_bond32t<4, 2, 0, 0>, 0);
+  set((const void *)k_bond32t<3, 4, 0, 1>, 0);
+  set((const void *)k_bond32t<4, 2, 0, 1>, 0);
+  set((const void *)k_bond32t<3, 4, 1, 0>, 1);
+  set((const void *)k_bond32t<4, 2, 1, 0>, 1);
+  set((const void *)k_bond32t<3, 4, 1, 1>, 1);
+  set((const void *)k_bond32t<4, 2, 1, 1>, 1);
+  return e;
 }
 
 // FP32 form: broken flags of the column entries from the live masks (after the masks were
@@ -1418,7 +1546,12 @@ __global__ void k_col_flags(const __grid_constant__ DevView v) {
   const int dg = v.deg[n];
   for (int j = 0; j < dg; ++j) {
     const uint32_t q = col[32 * j] & kColIndex;
-    col[32 * j] = ((maskp[j] >> lane) & 1u) ? q : (q | kColBroken);
+    const bool live = (maskp[j] >> lane) & 1u;
+    col[32 * j] = live ? q : (q | kColBroken);
+    if (v.tcol) {
+      uint16_t &t = v.tcol[tile_entry(sbase, (uint32_t)j, lane)];
+      t = live ? (uint16_t)(t & ~kTileBroken) : (uint16_t)(t | kTileBroken);
+    }
   }
 }
 
@@ -1483,23 +1616,30 @@ void launch_anchor_next(const DevView &v, cudaStream_t s) {
 
 // Bond-kernel variants the autotuner chooses from: k_bond32 <positions per load group, min
 // blocks/SM, 256-bit record loads, column prefetch, fused non-bond work> with 128-thread blocks
-// (0-9, 18-20) and with 32/64-thread blocks (14-17), the staged k_bond32s (10-13), k_bond32l with
+// (0-9, 18-20) and with 32/64-thread blocks (14-17), the tiled k_bond32t at 3 or 4
+// blocks/SM, without (10, 11) and with (12, 13) the non-bond work fused, k_bond32l with
 // 2 or 4 lanes per node (21-24) and k_bond32a, one lane per node gathering a group ahead (25-27).
 const int kNumBondVariants = 28;
 
 int num_bond_variants() { return kNumBondVariants; }
 
+template <int MINB, int U, int FX>
+static void launch_tile(const DevView &v, cudaStream_t s) {
+  const unsigned b = (unsigned)((v.N + kTileNodes - 1) / kTileNodes);
+  const size_t sm = (size_t)v.tile_max * tile_rec_bytes(v.tile_vol);
+  if (v.tile_vol) k_bond32t<MINB, U, 1, FX><<<b, kTileNodes, sm, s>>>(v);
+  else k_bond32t<MINB, U, 0, FX><<<b, kTileNodes, sm, s>>>(v);
+  if (v.tile_gather) k_bond32g<FX><<<b, kTileNodes, 0, s>>>(v);
+}
+
 void launch_step_fp32c(const DevView &v, int variant, cudaStream_t s) {
   const uint64_t blocks = (v.N + 127) / 128;
   if (!blocks) return;
   const unsigned b = (unsigned)blocks;
-  // nothing to stage (or the ranges not computed): the plain kernel
-  if (variant >= kFirstStagedVariant && variant < kFirstStagedVariant + 4 && !v.win_max) variant = 3;
-  const bool fused_extra = (variant >= 6 && variant <= 9) || (variant >= 14 && variant <= 16) || variant == 19 ||
+  if (variant >= kFirstTileVariant && variant <= kLastTileVariant && !v.tcol) variant = 18;  // no tiles built
+  const bool fused_extra = (variant >= 6 && variant <= 9) || (variant >= 12 && variant <= 16) || variant == 19 ||
                            variant >= 21;
   if (!fused_extra) k_extra32<<<152 * 8, 128, 0, s>>>(v);
-  const unsigned bs = (unsigned)((v.N + kStageNodes - 1) / kStageNodes);
-  const size_t sm = (size_t)v.win_max * sizeof(Rec32);
   switch (variant) {
     case 1: k_bond32<4, 6, 1, 1, 0><<<b, 128, 0, s>>>(v); break;
     case 2: k_bond32<4, 4, 1, 2, 0><<<b, 128, 0, s>>>(v); break;
@@ -1510,10 +1650,10 @@ void launch_step_fp32c(const DevView &v, int variant, cudaStream_t s) {
     case 7: k_bond32<4, 4, 1, 2, 1><<<b, 128, 0, s>>>(v); break;
     case 8: k_bond32<4, 6, 1, 1, 1><<<b, 128, 0, s>>>(v); break;
     case 9: k_bond32<4, 6, 1, 2, 1><<<b, 128, 0, s>>>(v); break;
-    case 10: k_bond32s<4, 1><<<bs, kStageNodes, sm, s>>>(v); break;
-    case 11: k_bond32s<4, 2><<<bs, kStageNodes, sm, s>>>(v); break;
-    case 12: k_bond32s<4, 3><<<bs, kStageNodes, sm, s>>>(v); break;
-    case 13: k_bond32s<8, 1><<<bs, kStageNodes, sm, s>>>(v); break;
+    case 10: launch_tile<3, 4, 0>(v, s); break;
+    case 11: launch_tile<4, 2, 0>(v, s); break;
+    case 12: launch_tile<3, 4, 1>(v, s); break;
+    case 13: launch_tile<4, 2, 1>(v, s); break;
     // small handles: a few hundred 128-thread blocks leave some SMs one block more than others;
     // 32- and 64-thread blocks of the same kernels spread the warps evenly
     case 14: k_bond32<4, 4, 1, 1, 1><<<(unsigned)((v.N + 31) / 32), 32, 0, s>>>(v); break;

@@ -47,7 +47,7 @@ __global__ void k_predict(DevView v) {
       inc2 = ix * ix + iy * iy + iz * iz;
       if (v.rec) {
         const double *an = v.anchor + 3 * (uint64_t)k;
-        v.rec[n].u = make_float4((float)(d.x - an[0]), (float)(d.y - an[1]), (float)(d.z - an[2]), 0.f);
+        set_rec_u(v.rec[n], (float)(d.x - an[0]), (float)(d.y - an[1]), (float)(d.z - an[2]));
       }
     }
   }
@@ -433,7 +433,7 @@ __global__ void k_prescribed(DevView v) {
       const D3 dn = d + inc;
       st3(v.disp_next, g, C3, dn);
       const double *anx = v.anchor_next + 3 * (uint64_t)k;
-      v.rec_next[g].u = make_float4((float)(dn.x - anx[0]), (float)(dn.y - anx[1]), (float)(dn.z - anx[2]), 0.f);
+      set_rec_u(v.rec_next[g], (float)(dn.x - anx[0]), (float)(dn.y - anx[1]), (float)(dn.z - anx[2]));
       const float ix = (float)(dn.x - d.x), iy = (float)(dn.y - d.y), iz = (float)(dn.z - d.z);
       i2 = fmaxf(i2, ix * ix + iy * iy + iz * iz);
     }
