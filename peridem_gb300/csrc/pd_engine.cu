@@ -583,7 +583,7 @@ int Engine::upload_bonds(SellHost &h) {
 
 int Engine::alloc_and_upload() {
   const uint64_t C = Ncap_;
-  constexpr uint64_t kChunk = 8192;  // nodes a host thread stages at a time
+  constexpr uint64_t kChunk = 16384;  // nodes a host thread stages at a time
   // The SELL-32 bond arrays: from a sorted Connectivity they are built on the device once the
   // node arrays (node_of among them) are uploaded, the bond counts being computed on a host
   // thread meanwhile; from any other Connectivity the whole build runs on a host thread beside

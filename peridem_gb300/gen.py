@@ -101,15 +101,18 @@ def bonds_gpu(positions: list, radii: list) -> list:
                                if P else np.zeros((0, 3)))
     rad = np.ascontiguousarray(radii, dtype=np.float64)
     po = np.zeros(P + 1, dtype=np.uint64)
-    rc = L.pd_query_pairs(ptr(pos), ptr(off), ptr(rad), P, None, 0, ptr(po))
+    # room for a lattice with a horizon of three spacings (54 pairs per node); where that is too
+    # little the call says how many pairs there are. Pages of `out` that no pair reaches are never touched
+    cap = 60 * len(pos) + 1024
+    out = np.empty((cap, 2), dtype=np.uint32)
+    rc = L.pd_query_pairs(ptr(pos), ptr(off), ptr(rad), P, ptr(out), cap, ptr(po))
+    if rc != 0 and int(po[-1]) > cap:
+        cap = int(po[-1])
+        out = np.empty((cap, 2), dtype=np.uint32)
+        rc = L.pd_query_pairs(ptr(pos), ptr(off), ptr(rad), P, ptr(out), cap, ptr(po))
     if rc != 0:
         raise RuntimeError(f"pd_query_pairs: [{rc}] {L.pd_pairs_error().decode()}")
-    M = int(po[-1])
-    out = np.zeros((max(M, 1), 2), dtype=np.uint32)
-    rc = L.pd_query_pairs(ptr(pos), ptr(off), ptr(rad), P, ptr(out), M, ptr(po))
-    if rc != 0:
-        raise RuntimeError(f"pd_query_pairs: [{rc}] {L.pd_pairs_error().decode()}")
-    return [out[int(po[p]):int(po[p + 1])].copy() for p in range(P)]
+    return [out[int(po[p]):int(po[p + 1])] for p in range(P)]
 
 
 def bonds(pos: np.ndarray, delta: float) -> np.ndarray:

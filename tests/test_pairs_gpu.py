@@ -150,3 +150,33 @@ def test_boundary_nodes_same_with_either_builder():
         gen.set_bond_builder("cpu")
     np.testing.assert_array_equal(cpu, gpu)
     assert 0 < len(cpu) < len(P)
+
+
+@pytest.mark.parametrize("case", ["dense", "far", "huge", "tiny", "row"])
+def test_edges_of_the_decision(case):
+    """Rows past the in-register sort's 128, a box of more than 1e6 cells (FP64 decides every pair),
+    radii whose square leaves the FP64 range, and points along one row of cells at spacings around
+    the radius."""
+    rng = np.random.default_rng(7)
+    r = {"huge": 1e180, "tiny": 1e-170}.get(case, 1e-4)
+    if case == "dense":
+        P = rng.uniform(0, 1e-4, (700, 3))
+    elif case == "far":
+        P = rng.uniform(0, 4e-4, (500, 3))
+        P[250:] += 3e3  # coordinates whose spacing is near r / 200
+    elif case == "row":
+        P = np.zeros((600, 3))
+        P[:, 0] = np.arange(600) * 0.5e-4 + rng.integers(-2, 3, 600) * np.spacing(0.5e-4)
+    else:
+        P = rng.uniform(0, r, (400, 3))
+    with np.errstate(over="ignore", under="ignore"):
+        np.testing.assert_array_equal(gen.bonds_gpu([P], [r])[0], _formula(P, r))
+        m = rng.random(len(P)) < 0.1
+        np.testing.assert_array_equal(gen.near_gpu([P], [m], [r])[0], _near_formula(P, m, r))
+
+
+def test_non_finite_position_is_refused():
+    P = np.zeros((4, 3))
+    P[2, 1] = np.nan
+    with pytest.raises(RuntimeError, match="non-finite"):
+        gen.bonds_gpu([P], [1e-4])
