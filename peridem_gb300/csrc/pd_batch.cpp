@@ -62,7 +62,9 @@ uint64_t Engine::estimate_bytes(const std::vector<HostSim> &sims, int precision,
   b += S * sizeof(DevSimParams) + S * sizeof(DevSimState) + sizeof(DevCounters);
   if (ncl) b += (P + 1 + ncl) * 4 + 3 * ncl * 8;
   if (precision == PD_FP64) {
-    b += 3 * atleast1(E) * 8 + 2 * atleast1(E) * 8;
+    uint64_t M = 0;
+    for (auto &s : sims) M += s.conn_offset[s.np];
+    b += atleast1(M) * (8 + 40 + sizeof(Pair64)) + atleast1(E) * 4 + atleast1(E / 32) * 4;
   } else {
     b += 2 * C * 32 + 3 * C * 8 + 2 * 3 * P * 8 + C + 3 * C * 8 + C + 2 * 6 * P * 4;
     const uint64_t nt = (N + kTileNodes - 1) / kTileNodes;

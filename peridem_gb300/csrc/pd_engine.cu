@@ -99,9 +99,12 @@ DevView Engine::view(int cur) const {
   v.deg = d_deg_;
   v.col = d_col_;
   v.mask = d_mask_;
-  v.bxi = d_bxi_;
-  v.bxin = d_bxin_;
-  v.brxin = d_brxin_;
+  v.M = M_;
+  v.pair_end = d_pair_end_;
+  v.pair_xi = d_pair_xi_;
+  v.pair = d_pair_;
+  v.pidx = d_pidx_;
+  v.plow = d_plow_;
   v.E = E_;
   v.anchor = d_anchor_;
   if (precision_ == PD_FP32C) {
@@ -573,6 +576,36 @@ int Engine::build_bonds_gpu(const std::vector<uint64_t> &rowptr, bool &fallback)
   return rc;
 }
 
+int Engine::build_pairs() {
+  M_ = initial_bonds_ / 2;  // every Connectivity row was pushed onto both of its ends
+  if (M_ > 0xFFFFFFFFull) {
+    err = "too many bonds for 32-bit pair indices";
+    return PD_EINVAL;
+  }
+  const uint64_t m = std::max<uint64_t>(M_, 1), ne = std::max<uint64_t>(E_, 1), nw = std::max<uint64_t>(E_ / 32, 1);
+  PD_TRY(dalloc(this, allocs_, &d_pair_end_, m, err));
+  PD_TRY(dalloc(this, allocs_, &d_pair_xi_, 5 * m, err));
+  PD_TRY(dalloc(this, allocs_, &d_pair_, m, err));
+  PD_TRY(dalloc(this, allocs_, &d_pidx_, ne, err));
+  PD_TRY(dalloc(this, allocs_, &d_plow_, nw, err));
+  uint32_t *first = nullptr, total = 0;  // scratch: [Ncap] first pairs, [Ncap] partner-side counts, the total
+  PD_TRY(check(cudaMallocAsync((void **)&first, (2 * Ncap_ + 1) * 4, stream_), "pair scratch"));
+  int rc = check(cudaMemsetAsync(first + 2 * Ncap_, 0, 4, stream_), "pair scratch");
+  if (rc == PD_OK) {
+    launch_pair_build(view(0), conn_sorted_, first, first + Ncap_, first + 2 * Ncap_, d_pair_end_, d_pair_xi_, d_pidx_,
+                      d_plow_, stream_);
+    rc = check(cudaGetLastError(), "pair build");
+  }
+  if (rc == PD_OK) rc = cpy(&total, first + 2 * Ncap_, 4, "pair count");
+  cudaFreeAsync(first, stream_);
+  PD_TRY(rc);
+  if (total != M_) {
+    err = "bond rows are not symmetric";
+    return PD_EINVAL;
+  }
+  return PD_OK;
+}
+
 int Engine::upload_bonds(SellHost &h) {
   const uint64_t ncol = h.ncol, nmask = h.nmask;
   PD_TRY(alloc_bond_arrays());
@@ -934,9 +967,7 @@ int Engine::alloc_and_upload() {
   }
 
   if (precision_ == PD_FP64) {
-    PD_TRY(dalloc(this, allocs_, &d_bxi_, 3 * std::max<uint64_t>(E_, 1), err));
-    PD_TRY(dalloc(this, allocs_, &d_bxin_, std::max<uint64_t>(E_, 1), err));
-    PD_TRY(dalloc(this, allocs_, &d_brxin_, std::max<uint64_t>(E_, 1), err));
+    PD_TRY(build_pairs());
   } else {
     std::unique_ptr<Rec32[]> r32(new Rec32[C]);  // every entry written below
     parallel_items((C + kChunk - 1) / kChunk, [&](uint64_t chunk) {
@@ -1005,7 +1036,6 @@ int Engine::alloc_and_upload() {
 
   if (precision_ == PD_FP64) {
     DevView v = view(0);
-    launch_bond_constants(v, d_bxi_, d_bxin_, d_brxin_, stream_);
     launch_init_lrtb(v, stream_);
     PD_TRY(check(cudaGetLastError(), "init kernels"));
   } else {

@@ -19,8 +19,9 @@
 //     FP32 kernels when they break the bond, re-derived from the masks after a restore or a
 //     set Connectivity), so that the FP32 bond loops read liveness with the column index;
 //     the masks stay the record every other reader uses;
-//   * FP64 form only: per-entry constants xi = pos[q]-pos[i] (3 doubles), |xi| and the
-//     correctly rounded reciprocal of |xi| (gen_xi, particle2.h:241-257);
+//   * FP64 form only: each bond once, owned by its end with the lower file index, with the
+//     constants xi = pos[q]-pos[i] (3 doubles), |xi| and the correctly rounded reciprocal of |xi|
+//     (gen_xi, particle2.h:241-257), and for every SELL entry the pair it belongs to;
 //   * FP32-compensated form only: a 32-byte record per node (Rec32: local position, local
 //     displacement, cnot * volume), double-buffered; local = relative to the particle's anchor node;
 //   * contact broad phase: hashed cell list (counting sort) rebuilt only when the nodes may
@@ -170,6 +171,12 @@ struct __align__(32) CellRec {
   uint32_t cx, cy, cz, sim;
 };
 
+// FP64 form: one bond's terms of a step, seen from its owner: stretch and unit vector. The other end's
+// are the same stretch and the negated vector, bit for bit.
+struct __align__(32) Pair64 {
+  double s, ux, uy, uz;
+};
+
 // Everything a kernel needs, passed by value.
 struct DevView {
   uint64_t N;            // nodes
@@ -190,8 +197,15 @@ struct DevView {
   const uint16_t *deg;
   const uint32_t *col;
   uint32_t *mask;
-  const double *bxi, *bxin, *brxin;  // FP64 form, [3][E], [E], [E]
   uint64_t E;
+  // FP64 form, the bonds as pairs (k_pair64): the owner and the partner of each of the M pairs, their
+  // constants xi, |xi|, RN(1/|xi|) ([5][M]) and this step's terms; per SELL entry the pair it is, and
+  // per (slice, position) the lanes whose entry is the partner's side
+  uint64_t M;
+  const uint2 *pair_end;
+  const double *pair_xi;
+  struct Pair64 *pair;
+  const uint32_t *pidx, *plow;
   // FP32-compensated form (the predictor of the next step runs in the bond kernel's tail:
   // disp/rec are read for this step while disp_next/rec_next receive the next one)
   Rec32 *rec, *rec_next;
@@ -538,7 +552,12 @@ class Engine {
   uint64_t *d_slice_ptr_ = nullptr;
   uint16_t *d_deg_ = nullptr;
   uint32_t *d_col_ = nullptr, *d_mask_ = nullptr;
-  double *d_bxi_ = nullptr, *d_bxin_ = nullptr, *d_brxin_ = nullptr;
+  uint64_t M_ = 0;  // FP64 form: pairs
+  uint2 *d_pair_end_ = nullptr;
+  double *d_pair_xi_ = nullptr;
+  Pair64 *d_pair_ = nullptr;
+  uint32_t *d_pidx_ = nullptr, *d_plow_ = nullptr;
+  int build_pairs();  // FP64 form, after the SELL arrays
   double *d_anchor_ = nullptr;
   double *d_f_extra_ = nullptr;
   uint32_t *d_tile_rec_ = nullptr, *d_tile_n_ = nullptr;
@@ -628,7 +647,10 @@ cudaError_t launch_tile_build(const DevView &v, uint32_t *tile_rec, uint32_t *ti
 void launch_end_step(const DevView &v, const uint32_t *clamped, uint64_t n_clamped, double *clamped_disp,
                      cudaStream_t s);
 void launch_centroids(const DevView &v, cudaStream_t s);
-void launch_bond_constants(const DevView &v, double *bxi, double *bxin, double *brxin, cudaStream_t s);
+// FP64 form: the pairs of the SELL rows. first[Ncap], low[Ncap]: scratch; *total (zeroed) receives the
+// number of pairs. sorted: every row is ascending in the file's numbering.
+void launch_pair_build(const DevView &v, bool sorted, uint32_t *first, uint32_t *low, uint32_t *total, uint2 *end,
+                       double *xi, uint32_t *pidx, uint32_t *plow, cudaStream_t s);
 void launch_broadphase(const DevView &v, BroadPhase &bp, cudaStream_t s);
 void launch_bp_decide(const DevView &v, double half_skin, cudaStream_t s, cudaGraphConditionalHandle cond = 0);
 void launch_pairwise_count(const DevView &v, cudaStream_t s);

@@ -66,6 +66,44 @@ void launch_predict(const DevView &v, int tpb, cudaStream_t s) {
 // ------------------------------------------------------------------------------------
 // fused force + corrector
 
+// A bond's terms are the same seen from both of its ends, but for the sign of the unit vector: every
+// operation on eta = (d_q - d_i) + xi is odd or even in it, rounding included. So each bond is
+// evaluated once (k_pair64), and k_step's rows add the terms in the reference's order: 27 FP64
+// instructions per row entry instead of 46 on a pipe that was 88 % busy (an FP64 instruction holds
+// it for 16 cycles of an SM a warp), and on small handles a bond per thread instead of a row's
+// square roots and divisions one after another.
+// crush512's 778k nodes, 7.0e7 row entries: MEASURED.
+__global__ void __launch_bounds__(256) k_pair64(const __grid_constant__ DevView v) {
+  const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= v.M) return;
+  const uint2 e = v.pair_end[k];
+  const DevPart &P = v.parts[v.pid[e.x]];
+  if (!P.movable || !v.ss[P.sim].active) return;
+  const D3 xi = ld3(v.pair_xi, k, v.M);
+  const D3 eta = (ld3(v.disp, e.y, v.Ncap) - ld3(v.disp, e.x, v.Ncap)) + xi;  // particle2.h:139-157
+  const double xn = v.pair_xi[k + 3 * v.M], rxn = v.pair_xi[k + 4 * v.M];
+  const double en = norm3(eta);
+  const double str = div_rcp(en - xn, xn, rxn);
+  const double ren = __drcp_rn(en);
+  const double ux = div_rcp(eta.x, en, ren), uy = div_rcp(eta.y, en, ren), uz = div_rcp(eta.z, en, ren);
+  asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(v.pair + k), "d"(str), "d"(ux), "d"(uy), "d"(uz)
+               : "memory");
+}
+
+// a > b for a positive finite b, by integer comparison (a NaN is not).
+__device__ __forceinline__ bool above(double a, long long b_bits) {
+  const long long x = __double_as_longlong(a);
+  return x > b_bits && x <= 0x7FF0000000000000ll;
+}
+
+// Least and largest of a warp's 64-bit keys.
+__device__ __forceinline__ unsigned long long warp_min_key(unsigned long long k) {
+  const uint32_t hi = __reduce_min_sync(0xffffffffu, (uint32_t)(k >> 32));
+  const uint32_t lo = __reduce_min_sync(0xffffffffu, (uint32_t)(k >> 32) == hi ? (uint32_t)k : 0xffffffffu);
+  return ((unsigned long long)hi << 32) | lo;
+}
+__device__ __forceinline__ unsigned long long warp_max_key(unsigned long long k) { return ~warp_min_key(~k); }
+
 __global__ void __launch_bounds__(128) k_step(DevView v) {
   const uint64_t n = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const bool valid = n < v.N;
@@ -94,22 +132,38 @@ __global__ void __launch_bounds__(128) k_step(DevView v) {
     const int dg = v.deg[nn];
     const bool brk = st.fracture && P.breakable && P.break_bonds;
     D3 acc = d3(0.0, 0.0, 0.0);
-    for (int j = 0; j < dg; ++j) {
-      const uint32_t mw = v.mask[mbase + j];
-      if (!((mw >> lane) & 1u)) continue;
-      const uint64_t e = base + 32ull * j;
-      const uint32_t q = v.col[e];
-      ++live;
-      D3 dq = ld3(v.disp, q, C3);
-      D3 eta = (dq - di) + d3(v.bxi[e], v.bxi[e + v.E], v.bxi[e + 2 * v.E]);
-      double en = norm3(eta);
-      double xn = v.bxin[e];
-      double str = div_rcp(en - xn, xn, v.brxin[e]);
-      double mag = (P.cnot * str) * v.vol[q];
-      double ren = __drcp_rn(en);
-      D3 unit = d3(div_rcp(eta.x, en, ren), div_rcp(eta.y, en, ren), div_rcp(eta.z, en, ren));
-      acc = acc + mag * unit;
-      if (brk && str > P.snot) atomicAnd(&v.mask[mbase + j], ~(1u << lane));
+    const bool pos_snot = P.snot > 0 && isfinite(P.snot);
+    const long long snot_bits = __double_as_longlong(P.snot);
+    // four entries' terms requested at once, added in row order
+    for (int j0 = 0; j0 < dg; j0 += 4) {
+      uint32_t mw[4], lw[4], id[4], q[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const bool in = j0 + u < dg;
+        const uint64_t e = base + 32ull * (j0 + u);
+        mw[u] = in ? v.mask[mbase + j0 + u] : 0u;
+        lw[u] = in ? v.plow[mbase + j0 + u] : 0u;
+        id[u] = in ? v.pidx[e] : 0u;
+        q[u] = in ? v.col[e] : (uint32_t)nn;
+      }
+      double s[4], ux[4], uy[4], uz[4], vol[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+            : "=d"(s[u]), "=d"(ux[u]), "=d"(uy[u]), "=d"(uz[u])
+            : "l"(v.pair + id[u]));
+        vol[u] = v.vol[q[u]];
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (!((mw[u] >> lane) & 1u)) continue;
+        ++live;
+        double mag = (P.cnot * s[u]) * vol[u];
+        // the partner's side: the unit vector negated, here as the sign of its factor
+        mag = __hiloint2double(__double2hiint(mag) ^ (int)(((lw[u] >> lane) & 1u) << 31), __double2loint(mag));
+        acc = acc + mag * d3(ux[u], uy[u], uz[u]);
+        if (brk && (pos_snot ? above(s[u], snot_bits) : s[u] > P.snot)) atomicAnd(&v.mask[mbase + j0 + u], ~(1u << lane));
+      }
     }
     f = d3(0.0, 0.0, 0.0) + acc;
 
@@ -235,7 +289,7 @@ __global__ void __launch_bounds__(128) k_step(DevView v) {
   // ---- corrector (timeloop.h:662-781)
   if (run) {
     st3(v.force, nn, C3, f);
-    if (!(isfinite(f.x) && isfinite(f.y) && isfinite(f.z))) atomicOr(&v.cnt->err, PD_DERR_NONFINITE);
+    if (nonfinite(f.x) || nonfinite(f.y) || nonfinite(f.z)) atomicOr(&v.cnt->err, PD_DERR_NONFINITE);
     D3 vo = vi;
     if (P.movable) {
       const D3 ao = ld3(v.acc, nn, C3);
@@ -249,28 +303,33 @@ __global__ void __launch_bounds__(128) k_step(DevView v) {
     st3(v.vel_out, nn, C3, vo);
   }
 
-  // ---- AABB of CurrPos for the next step (timeloop.h:779), warp-reduced
+  // ---- AABB of CurrPos for the next step (timeloop.h:779), warp-reduced as ordered keys (integer
+  // instructions: FP64 comparisons share the pipe with the bond terms); a NaN coordinate counts as
+  // absent
   {
     const bool contrib = run && P.movable;
-    D3 cur = pi + di;
-    double lo[3] = {contrib ? cur.x : INFINITY, contrib ? cur.y : INFINITY, contrib ? cur.z : INFINITY};
-    double hi[3] = {contrib ? cur.x : -INFINITY, contrib ? cur.y : -INFINITY, contrib ? cur.z : -INFINITY};
+    const D3 cur = pi + di;
+    unsigned long long lo[3], hi[3];
+    for (int c = 0; c < 3; ++c) {
+      const double x = comp(cur, c);
+      const bool on = contrib && !((__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFll) > 0x7FF0000000000000ll);
+      lo[c] = ord_key(on ? x : INFINITY);
+      hi[c] = ord_key(on ? x : -INFINITY);
+    }
     const uint32_t k0 = __shfl_sync(0xffffffffu, k, 0);
     const bool uniform = __all_sync(0xffffffffu, k == k0);
     if (uniform) {
-      for (int o = 16; o > 0; o >>= 1) {
-        for (int c = 0; c < 3; ++c) {
-          lo[c] = fmin(lo[c], __shfl_xor_sync(0xffffffffu, lo[c], o));
-          hi[c] = fmax(hi[c], __shfl_xor_sync(0xffffffffu, hi[c], o));
-        }
+      for (int c = 0; c < 3; ++c) {
+        lo[c] = warp_min_key(lo[c]);
+        hi[c] = warp_max_key(hi[c]);
       }
     }
     const bool writer = uniform ? ((threadIdx.x & 31) == 0) : contrib;
     if (writer && lo[0] <= hi[0]) {
       unsigned long long *L = reinterpret_cast<unsigned long long *>(v.lrtb_next) + 6 * (uint64_t)k;
       for (int c = 0; c < 3; ++c) {
-        atomicMin(&L[c], ord_key(lo[c]));
-        atomicMax(&L[3 + c], ord_key(hi[c]));
+        atomicMin(&L[c], lo[c]);
+        atomicMax(&L[3 + c], hi[c]);
       }
     }
   }
@@ -290,10 +349,12 @@ __global__ void __launch_bounds__(128) k_step(DevView v) {
 void launch_step_kernel(const DevView &v, int precision, int variant, cudaStream_t s) {
   uint64_t blocks = (v.N + 127) / 128;
   if (!blocks) return;
-  if (precision == PD_FP32C)
+  if (precision == PD_FP32C) {
     launch_step_fp32c(v, variant, s);
-  else
-    k_step<<<(unsigned)blocks, 128, 0, s>>>(v);
+    return;
+  }
+  if (v.M) k_pair64<<<(unsigned)((v.M + 255) / 256), 256, 0, s>>>(v);
+  k_step<<<(unsigned)blocks, 128, 0, s>>>(v);
 }
 
 // ------------------------------------------------------------------------------------
@@ -536,31 +597,118 @@ void launch_reset_y(const DevView &v, cudaStream_t s) {
   if (v.S) k_reset_y<<<v.S, 256, 0, s>>>(v);
 }
 
-// gen_xi (particle2.h:241-257): xi = pos[q] - pos[i], |xi| and RN(1/|xi|) per SELL entry.
-__global__ void k_bond_constants(DevView v, double *bxi, double *bxin, double *brxin) {
+// The pairs of the FP64 form. The end with the lower file index owns a bond; of a bond of a node with
+// itself, pushed twice onto its row, the first entry does. A node's pairs lie one after another in
+// row order, the nodes of a block in order, the blocks in the order they finish counting (a pair's
+// place does not matter to any result).
+__global__ void __launch_bounds__(256) k_pair_count(const __grid_constant__ DevView v, uint32_t *first, uint32_t *low,
+                                                    uint32_t *total) {
   const uint64_t n = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= v.N) return;
-  const uint64_t s = n >> 5;
-  const uint32_t lane = (uint32_t)(n & 31);
-  const uint64_t base = v.slice_ptr[s] + lane;
-  const D3 pi = ld3(v.pos, n, v.Ncap);
-  const int dg = v.deg[n];
-  for (int j = 0; j < dg; ++j) {
-    const uint64_t e = base + 32ull * j;
-    const uint32_t q = v.col[e];
-    D3 xi = ld3(v.pos, q, v.Ncap) - pi;
-    double xn = norm3(xi);
-    bxi[e] = xi.x;
-    bxi[e + v.E] = xi.y;
-    bxi[e + 2 * v.E] = xi.z;
-    bxin[e] = xn;
-    brxin[e] = __drcp_rn(xn);
+  uint32_t own = 0, other = 0;
+  if (n < v.N) {
+    const uint32_t *row = v.col + v.slice_ptr[n >> 5] + (n & 31);
+    const uint32_t fn = v.file_of[n];
+    const int dg = v.deg[n];
+    bool again = false;
+    for (int j = 0; j < dg; ++j) {
+      const uint32_t q = row[32 * j];
+      const bool mine = q == n ? !again : v.file_of[q] > fn;
+      if (q == n) again = !again;
+      mine ? ++own : ++other;
+    }
+  }
+  __shared__ uint32_t warps[8], base;
+  const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  uint32_t s = own;
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, s, o);
+    if (lane >= (uint32_t)o) s += y;
+  }
+  if (lane == 31) warps[w] = s;
+  __syncthreads();
+  uint32_t before = 0, sum = 0;
+  for (uint32_t i = 0; i < 8; ++i) {
+    if (i < w) before += warps[i];
+    sum += warps[i];
+  }
+  if (threadIdx.x == 0) base = atomicAdd(total, sum);
+  __syncthreads();
+  if (n < v.N) {
+    first[n] = base + before + s - own;
+    low[n] = other;
   }
 }
 
-void launch_bond_constants(const DevView &v, double *bxi, double *bxin, double *brxin, cudaStream_t s) {
-  uint64_t blocks = (v.N + 127) / 128;
-  if (blocks) k_bond_constants<<<(unsigned)blocks, 128, 0, s>>>(v, bxi, bxin, brxin);
+// gen_xi (particle2.h:241-257) for the owned pairs: xi = pos[q] - pos[i], |xi| and RN(1/|xi|); every
+// entry's pair: an owner's its own, another's the one its partner's row holds for it.
+__global__ void __launch_bounds__(256) k_pair_fill(const __grid_constant__ DevView v, bool sorted,
+                                                   const uint32_t *first, const uint32_t *low, uint2 *end, double *xi,
+                                                   uint32_t *pidx, uint32_t *plow) {
+  const uint64_t n = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;  // whole warps: Ncap is a multiple of 32
+  if (n >= v.Ncap) return;
+  const uint32_t lane = (uint32_t)(n & 31);
+  const uint64_t base = v.slice_ptr[n >> 5];
+  const int dg = n < v.N ? v.deg[n] : 0, w = (int)((v.slice_ptr[(n >> 5) + 1] - base) >> 5);
+  const uint32_t fn = n < v.N ? v.file_of[n] : 0u;
+  const D3 pi = ld3(v.pos, n, v.Ncap);
+  uint32_t k = n < v.N ? first[n] : 0u;
+  uint32_t again = 0, self = 0;
+  for (int j = 0; j < w; ++j) {
+    const uint64_t e = base + 32ull * j + lane;
+    bool theirs = false;
+    if (j < dg) {
+      const uint32_t q = v.col[e];
+      const uint32_t fq = v.file_of[q];
+      if (q == n ? !again : fq > fn) {
+        const D3 x = ld3(v.pos, q, v.Ncap) - pi;
+        const double xn = norm3(x);
+        end[k] = make_uint2((uint32_t)n, q);
+        xi[k] = x.x;
+        xi[k + v.M] = x.y;
+        xi[k + 2 * v.M] = x.z;
+        xi[k + 3 * v.M] = xn;
+        xi[k + 4 * v.M] = __drcp_rn(xn);
+        if (q == n) self = k;
+        pidx[e] = k++;
+      } else if (q == n) {
+        theirs = true;
+        pidx[e] = self;
+      } else {
+        theirs = true;
+        const uint32_t *row = v.col + v.slice_ptr[q >> 5] + (q & 31);
+        const int dq = v.deg[q];
+        uint32_t at = 0;
+        if (sorted) {  // the row ascends by file index, the entries q owns last
+          int a = 0, b = dq;
+          while (b - a > 1) {
+            const int m = (a + b) >> 1;
+            if (v.file_of[row[32 * m]] <= fn) a = m;
+            else b = m;
+          }
+          at = (uint32_t)a - low[q];
+        } else {  // the owned entries before it
+          bool twice = false;
+          for (int m = 0; m < dq && row[32 * m] != n; ++m) {
+            const uint32_t c = row[32 * m];
+            at += (c == q ? !twice : v.file_of[c] > fq) ? 1u : 0u;
+            if (c == q) twice = !twice;
+          }
+        }
+        pidx[e] = first[q] + at;
+      }
+      if (q == n) again ^= 1u;
+    } else {
+      pidx[e] = 0;
+    }
+    const uint32_t bits = __ballot_sync(0xffffffffu, theirs);
+    if (lane == 0) plow[(base >> 5) + j] = bits;
+  }
+}
+
+void launch_pair_build(const DevView &v, bool sorted, uint32_t *first, uint32_t *low, uint32_t *total, uint2 *end,
+                       double *xi, uint32_t *pidx, uint32_t *plow, cudaStream_t s) {
+  k_pair_count<<<(unsigned)((v.N + 255) / 256), 256, 0, s>>>(v, first, low, total);
+  k_pair_fill<<<(unsigned)((v.Ncap + 255) / 256), 256, 0, s>>>(v, sorted, first, low, end, xi, pidx, plow);
 }
 
 // AABBs of all particles before the loop (timeloop.h:389-393). A warp whose nodes all belong to
