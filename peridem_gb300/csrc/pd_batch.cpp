@@ -69,7 +69,7 @@ uint64_t Engine::estimate_bytes(const std::vector<HostSim> &sims, int precision,
     b += 2 * C * 32 + 3 * C * 8 + 2 * 3 * P * 8 + C + 3 * C * 8 + C + 2 * 6 * P * 4;
     const uint64_t nt = (N + kTileNodes - 1) / kTileNodes;
     if (N >= kTileMinNodes) b += nt * kTileRecords * 4 + nt * 4 + atleast1(E) * 2;  // tile arrays
-    b += C * 4 + atleast1(P) * 4 + 2 * 4;                          // non-bond work lists
+    b += atleast1(P) * 4;  // particles with non-bond work
   }
   // broad phase
   uint32_t bits = 10;
@@ -77,6 +77,7 @@ uint64_t Engine::estimate_bytes(const std::vector<HostSim> &sims, int precision,
   const uint64_t T = 1ull << bits;
   b += (2 * T + 1) * 4 + 2 * C * 4 + C * sizeof(CellRec) + ((T + 4095) / 4096 + 1) * 4;
   b += C * (cand_cap ? cand_cap : 32) * 4 + C * 2;
+  b += C * 4 + 2 * 4;  // nodes with contact candidates
   return b;
 }
 

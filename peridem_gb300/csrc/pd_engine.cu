@@ -1026,12 +1026,10 @@ int Engine::alloc_and_upload() {
   PD_TRY(dalloc(this, allocs_, &bp_.slot, C, err));
   PD_TRY(dalloc(this, allocs_, &bp_.rec, C, err));
   PD_TRY(dalloc(this, allocs_, &bp_.block_sums, (T + 4095) / 4096 + 1, err));
-  if (precision_ == PD_FP32C) {
-    PD_TRY(dalloc(this, allocs_, &bp_.xnodes, C, err));
-    PD_TRY(dalloc(this, allocs_, &bp_.xparts, P_, err));
-    PD_TRY(dalloc(this, allocs_, &bp_.xcount, 2, err));
-    PD_TRY(mset(bp_.xcount, 0, 8, "work lists"));
-  }
+  PD_TRY(dalloc(this, allocs_, &bp_.xnodes, C, err));
+  if (precision_ == PD_FP32C) PD_TRY(dalloc(this, allocs_, &bp_.xparts, P_, err));
+  PD_TRY(dalloc(this, allocs_, &bp_.xcount, 2, err));
+  PD_TRY(mset(bp_.xcount, 0, 8, "work lists"));
   PD_TRY(alloc_candidates());
 
   if (precision_ == PD_FP64) {
@@ -1840,7 +1838,7 @@ int Engine::snapshot() {
   }
   // the contact candidate lists, the cell list and the FP32 form's contact-node list are
   // derived from the positions: restore() has the next step rebuild them instead
-  if (bp_.xcount) {
+  if (bp_.xparts) {
     reg(bp_.xparts, (size_t)P_ * 4);
     reg(bp_.xcount, 8);
   }

@@ -268,7 +268,7 @@ struct BroadPhase {
   uint16_t *cand_n = nullptr;
   uint32_t cand_cap = 0;
   double skin_frac = 0.5;
-  // FP32 form: the nodes that have contact candidates (rebuilt with the lists), the particles
+  // the nodes that have contact candidates (rebuilt with the lists), in the FP32 form the particles
   // that need FP64 non-bond work next step, and their counts ([0] nodes, [1] particles)
   uint32_t *xnodes = nullptr, *xparts = nullptr, *xcount = nullptr;
 };

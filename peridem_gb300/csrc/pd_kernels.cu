@@ -20,6 +20,7 @@
 #include "pd_device.cuh"
 #include "pd_end.cuh"
 #include "pd_engine.h"
+#include "pd_extra.cuh"
 #include "pd_math.cuh"
 
 namespace pdg {
@@ -72,7 +73,9 @@ void launch_predict(const DevView &v, int tpb, cudaStream_t s) {
 // instructions per row entry instead of 46 on a pipe that was 88 % busy (an FP64 instruction holds
 // it for 16 cycles of an SM a warp), and on small handles a bond per thread instead of a row's
 // square roots and divisions one after another.
-// crush512's 778k nodes, 7.0e7 row entries: MEASURED.
+// 778k nodes, 7.0e7 row entries: 6.1 ms in one kernel; now 2.2 ms here (the FP64 pipe) and 1.25 ms in
+// k_step. 8,338 nodes: 257 us; now 30 us here and 56 us in k_step (and 13-39 in
+// k_contact64).
 __global__ void __launch_bounds__(256) k_pair64(const __grid_constant__ DevView v) {
   const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= v.M) return;
@@ -104,12 +107,49 @@ __device__ __forceinline__ unsigned long long warp_min_key(unsigned long long k)
 }
 __device__ __forceinline__ unsigned long long warp_max_key(unsigned long long k) { return ~warp_min_key(~k); }
 
+// Velocity-Verlet corrector of a node, given its whole force density (timeloop.h:662-781).
+__device__ __forceinline__ void correct64(const DevView &v, uint64_t nn, uint32_t k, const DevPart &P,
+                                          const DevSimParams &sp, const DevSimState &st, D3 vi, D3 f) {
+  const uint64_t C3 = v.Ncap;
+  const D3 ao = ld3(v.acc, nn, C3);
+  D3 vo = vi;
+  st3(v.force, nn, C3, f);
+  if (nonfinite(f.x) || nonfinite(f.y) || nonfinite(f.z)) atomicOr(&v.cnt->err, PD_DERR_NONFINITE);
+  if (P.movable) {
+    if (v.afd && st.vconstraint && (int32_t)(k - sp.p0) == sp.pv_particle) st3(v.afd, nn, C3, ao);
+    const D3 an = P.irho * f;
+    D3 tmp = ao + an;
+    tmp = sp.hdt * tmp;
+    vo = vi + tmp;
+    st3(v.acc, nn, C3, an);
+  }
+  st3(v.vel_out, nn, C3, vo);
+}
+
+// Node-level inputs of the non-bond force in this form: every movable node takes the walls' exact
+// tests and its external force.
+__device__ __forceinline__ ExtraCtx ctx64(const DevView &v, uint64_t n, uint32_t k, const DevPart &P,
+                                          const DevSimParams &sp, D3 pi, D3 di, D3 vi) {
+  ExtraCtx c;
+  c.k = k;
+  c.nc = v.cand_n[n] != 0;
+  c.mov = P.movable != 0;
+  c.wall_near = P.stoppable && sp.allow_wall;
+  c.ext = c.mov;
+  c.di = di;
+  c.pi = pi;
+  c.vi = vi;
+  c.voli = v.vol[n];
+  c.bdry_i = v.bdry[n] != 0;
+  return c;
+}
+
 __global__ void __launch_bounds__(128) k_step(DevView v) {
   const uint64_t n = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const bool valid = n < v.N;
   const uint64_t nn = valid ? n : 0;
   const uint32_t k = v.pid[nn];
-  const DevPart P = v.parts[k];
+  const DevPart &P = v.parts[k];
   const DevSimParams &sp = v.sp[P.sim];
   DevSimState &st = v.ss[P.sim];
   const bool run = valid && st.active;
@@ -119,9 +159,7 @@ __global__ void __launch_bounds__(128) k_step(DevView v) {
   D3 di = ld3(v.disp, nn, C3);
   const D3 pi = ld3(v.pos, nn, C3);
   const D3 vi = ld3(v.vel_in, nn, C3);
-  const double voli = v.vol[nn];
-  const bool bdry_i = v.bdry[nn] != 0;
-  unsigned long long live = 0, ncontacts = 0;
+  unsigned long long live = 0;
 
   if (run && P.movable) {
     // ---- peridynamic bond force (particle2.h:117-157) and breaking (particle2.h:196-237)
@@ -134,173 +172,76 @@ __global__ void __launch_bounds__(128) k_step(DevView v) {
     D3 acc = d3(0.0, 0.0, 0.0);
     const bool pos_snot = P.snot > 0 && isfinite(P.snot);
     const long long snot_bits = __double_as_longlong(P.snot);
-    // four entries' terms requested at once, added in row order
-    for (int j0 = 0; j0 < dg; j0 += 4) {
-      uint32_t mw[4], lw[4], id[4], q[4];
+    // four entries at a time, added in row order; the terms of the next four and the indices of the
+    // four after them are requested before these are added
+    struct Index {
+      uint32_t mw, lw, id, q;
+    };
+    struct Terms {
+      double s, x, y, z, vol;
+    };
+    auto index = [&](int j) {
+      const bool in = j < dg;
+      const uint64_t e = base + 32ull * j;
+      return Index{in ? v.mask[mbase + j] : 0u, in ? v.plow[mbase + j] : 0u, in ? v.pidx[e] : 0u,
+                   in ? v.col[e] : (uint32_t)nn};
+    };
+    auto terms = [&](const Index &i) {
+      Terms t;
+      asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+          : "=d"(t.s), "=d"(t.x), "=d"(t.y), "=d"(t.z)
+          : "l"(v.pair + i.id));
+      t.vol = v.vol[i.q];
+      return t;
+    };
+    constexpr int U = 4;
+    Index now[U], next[U];
+    Terms tn[U];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const bool in = j0 + u < dg;
-        const uint64_t e = base + 32ull * (j0 + u);
-        mw[u] = in ? v.mask[mbase + j0 + u] : 0u;
-        lw[u] = in ? v.plow[mbase + j0 + u] : 0u;
-        id[u] = in ? v.pidx[e] : 0u;
-        q[u] = in ? v.col[e] : (uint32_t)nn;
-      }
-      double s[4], ux[4], uy[4], uz[4], vol[4];
+    for (int u = 0; u < U; ++u) now[u] = index(u);
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
-            : "=d"(s[u]), "=d"(ux[u]), "=d"(uy[u]), "=d"(uz[u])
-            : "l"(v.pair + id[u]));
-        vol[u] = v.vol[q[u]];
-      }
+    for (int u = 0; u < U; ++u) next[u] = index(U + u);
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        if (!((mw[u] >> lane) & 1u)) continue;
+    for (int u = 0; u < U; ++u) tn[u] = terms(now[u]);
+    for (int j0 = 0; j0 < dg; j0 += U) {
+      Terms t[U];
+      Index after[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) t[u] = tn[u];
+#pragma unroll
+      for (int u = 0; u < U; ++u) tn[u] = terms(next[u]);
+#pragma unroll
+      for (int u = 0; u < U; ++u) after[u] = index(j0 + 2 * U + u);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (!((now[u].mw >> lane) & 1u)) continue;
         ++live;
-        double mag = (P.cnot * s[u]) * vol[u];
+        double mag = (P.cnot * t[u].s) * t[u].vol;
         // the partner's side: the unit vector negated, here as the sign of its factor
-        mag = __hiloint2double(__double2hiint(mag) ^ (int)(((lw[u] >> lane) & 1u) << 31), __double2loint(mag));
-        acc = acc + mag * d3(ux[u], uy[u], uz[u]);
-        if (brk && (pos_snot ? above(s[u], snot_bits) : s[u] > P.snot)) atomicAnd(&v.mask[mbase + j0 + u], ~(1u << lane));
+        mag = __hiloint2double(__double2hiint(mag) ^ (int)(((now[u].lw >> lane) & 1u) << 31), __double2loint(mag));
+        acc = acc + mag * d3(t[u].x, t[u].y, t[u].z);
+        if (brk && (pos_snot ? above(t[u].s, snot_bits) : t[u].s > P.snot))
+          atomicAnd(&v.mask[mbase + j0 + u], ~(1u << lane));
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        now[u] = next[u];
+        next[u] = after[u];
       }
     }
     f = d3(0.0, 0.0, 0.0) + acc;
-
-    // ---- self-contact (timeloop.h:554-557, contact.h:779-796), C side only
-    if (st.fracture && P.breakable && st.self_contact && (!sp.nl_bdry_only || bdry_i)) {
-      CandWalk walk(v, nn);
-      uint32_t m;
-      while (walk.next(m)) {
-        if (m < P.g0) continue;
-        if (m >= P.g0 + P.n) break;
-        if (sp.nl_bdry_only && !v.bdry[m]) continue;
-        D3 xi = ld3(v.pos, m, C3) - pi;
-        D3 dir = (ld3(v.disp, m, C3) - di) + xi;
-        const double q = sq3(dir);
-        if (q >= sp.rc2_far) continue;  // outside Rc for certain: skip the square root
-        double dn = sqrt(q);
-        if (!(dn <= sp.Rc)) continue;
-        double xin = norm3(xi);
-        double len_ref = sp.Rc, sc = sp.sc;
-        if (row_has_live(v, nn, m)) continue;
-        if (xin < sp.Rc) {
-          len_ref = xin;
-          sc = P.cnot;
-        }
-        if (!(dn < len_ref)) continue;
-        PairForce pf;
-        pair_force(dir, dn, len_ref, sc, v.vol[m], P.rho, vi, ld3(v.vel_in, m, C3), sp, st, pf);
-        if (P.stoppable) {
-          f = f + pf.fc;
-          if (pf.has_fd) f = f + pf.fd;
-          if (pf.has_ff) f = f + pf.ff;
-        }
-      }
-    }
-
-    // ---- walls (timeloop.h:561-569, contact.h:1094-1121)
-    if (P.stoppable && sp.allow_wall && !within_interior(v.lrtb + 6 * (uint64_t)k, st.wall, sp.Rc) &&
-        (!sp.nl_bdry_only || bdry_i)) {
-      D3 cur = pi + di;
-      const bool rx = sp.compute_wall_reaction != 0;
-      wall_face(cur.x - st.wall[0], 0, vi, voli, P.rho, f, st.spd[0], 0, sp, st, rx);
-      wall_face(cur.x - st.wall[3], 0, vi, voli, P.rho, f, st.spd[3], 3, sp, st, rx);
-      wall_face(cur.y - st.wall[1], 1, vi, voli, P.rho, f, st.spd[1], 1, sp, st, rx);
-      wall_face(cur.y - st.wall[4], 1, vi, voli, P.rho, f, st.spd[4], 4, sp, st, rx);
-      wall_face(cur.z - st.wall[2], 2, vi, voli, P.rho, f, st.spd[2], 2, sp, st, rx);
-      wall_face(cur.z - st.wall[5], 2, vi, voli, P.rho, f, st.spd[5], 5, sp, st, rx);
-    }
-
-    // ---- external force (timeloop.h:582-597)
-    D3 ex = ld3(v.ext, nn, C3);
-    if (sp.gradient_extforce) ex = st.extf_scale * ex;
-    f = f + ex;
   }
 
-  // ---- torque about the centroid (timeloop.h:600-633), for movable and fixed particles
-  if (run && st.torque) {
-    const double *c = v.centroid + 3 * (uint64_t)k;
-    D3 r = (pi + di) - d3(c[0], c[1], c[2]);
-    double rn = norm3(r);
-    double r_inv = (rn != 0.0 ? 1 / rn : 0);
-    const int ta = (int)P.taxis;
-    set_comp(r, ta, 0.0);
-    D3 perp = d3(0.0, 0.0, 0.0);
-    set_comp(perp, (ta + 1) % 3, -comp(r, (ta + 2) % 3));
-    set_comp(perp, (ta + 2) % 3, comp(r, (ta + 1) % 3));
-    double pn = norm3(perp);
-    if (pn > 0) {
-      perp = perp / pn;
-    } else {
-      set_comp(perp, (ta + 1) % 3, 0.0);
-      set_comp(perp, (ta + 2) % 3, 0.0);
-    }
-    f = f + (r_inv * P.tval) * perp;
-  }
-
-  // ---- node-node contact of particle pairs (timeloop.h:636-651, contact.h:754-937):
-  // partners in ascending file-order global index; a partner in a lower particle index acts as
-  // the "C" node of the pair (reaction form), a partner in a higher index as the "N" node.
-  if (run && P.stoppable && (!sp.nl_bdry_only || bdry_i)) {
-    CandWalk walk(v, nn);
-    uint32_t m;
-    while (walk.next(m)) {
-      if (m >= P.g0 && m < P.g0 + P.n) continue;
-      const uint32_t km = v.pid[m];
-      const uint32_t a = km < k ? km : k, b = km < k ? k : km;
-      if (!(v.parts[a].movable || v.parts[b].movable)) continue;
-      if (!intersects_fext(v.lrtb + 6 * (uint64_t)a, v.lrtb + 6 * (uint64_t)b, sp.Rc)) continue;
-      if (sp.nl_bdry_only && !v.bdry[m]) continue;
-      const D3 pm = ld3(v.pos, m, C3), dm = ld3(v.disp, m, C3), vm = ld3(v.vel_in, m, C3);
-      const double volm = v.vol[m];
-      if (km > k) {
-        D3 xi = pm - pi;
-        D3 dir = (dm - di) + xi;
-        const double q = sq3(dir);
-        if (q >= sp.rc2_far) continue;
-        double dn = sqrt(q);
-        if (!(dn <= sp.Rc) || !(dn < sp.Rc)) continue;
-        PairForce pf;
-        pair_force(dir, dn, sp.Rc, sp.sc, volm, P.rho, vi, vm, sp, st, pf);
-        f = f + pf.fc;
-        if (pf.has_fd) f = f + pf.fd;
-        if (pf.has_ff) f = f + pf.ff;
-        ++ncontacts;
-      } else {
-        D3 xi = pi - pm;
-        D3 dir = (di - dm) + xi;
-        const double q = sq3(dir);
-        if (q >= sp.rc2_far) continue;
-        double dn = sqrt(q);
-        if (!(dn <= sp.Rc) || !(dn < sp.Rc)) continue;
-        PairForce pf;
-        pair_force(dir, dn, sp.Rc, sp.sc, voli, v.parts[km].rho, vm, vi, sp, st, pf);
-        f = f - (pf.fc / voli) * volm;
-        if (pf.has_fd) {
-          double sn = sqrt(voli), sv = sqrt(volm);
-          f = f - (pf.fd / sn) * sv;
-        }
-        if (pf.has_ff) f = f - pf.ff;
-      }
-    }
-  }
-
-  // ---- corrector (timeloop.h:662-781)
+  // walls, external force and torque, then the corrector. A node with contact candidates leaves its
+  // bond sum to k_contact64 instead: its pairs are chains of FP64 square roots and divisions, ~5 us
+  // each, on which the node's whole warp and then the kernel would wait.
   if (run) {
-    st3(v.force, nn, C3, f);
-    if (nonfinite(f.x) || nonfinite(f.y) || nonfinite(f.z)) atomicOr(&v.cnt->err, PD_DERR_NONFINITE);
-    D3 vo = vi;
-    if (P.movable) {
-      const D3 ao = ld3(v.acc, nn, C3);
-      if (v.afd && st.vconstraint && (int32_t)(k - sp.p0) == sp.pv_particle) st3(v.afd, nn, C3, ao);
-      const D3 an = P.irho * f;
-      D3 tmp = ao + an;
-      tmp = sp.hdt * tmp;
-      vo = vi + tmp;
-      st3(v.acc, nn, C3, an);
+    if (v.cand_n[nn] != 0) {
+      st3(v.force, nn, C3, f);
+    } else {
+      extra_middle(v, nn, P, sp, st, ctx64(v, nn, k, P, sp, pi, di, vi), f);
+      correct64(v, nn, k, P, sp, st, vi, f);
     }
-    st3(v.vel_out, nn, C3, vo);
   }
 
   // ---- AABB of CurrPos for the next step (timeloop.h:779), warp-reduced as ordered keys (integer
@@ -335,14 +276,30 @@ __global__ void __launch_bounds__(128) k_step(DevView v) {
   }
 
   if (v.stats) {
-    for (int o = 16; o > 0; o >>= 1) {
-      live += __shfl_xor_sync(0xffffffffu, live, o);
-      ncontacts += __shfl_xor_sync(0xffffffffu, ncontacts, o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-      if (live) atomicAdd(&v.cnt->live_bonds, live);
-      if (ncontacts) atomicAdd(&v.cnt->contacts, ncontacts);
-    }
+    for (int o = 16; o > 0; o >>= 1) live += __shfl_xor_sync(0xffffffffu, live, o);
+    if ((threadIdx.x & 31) == 0 && live) atomicAdd(&v.cnt->live_bonds, live);
+  }
+}
+
+// The nodes with contact candidates (listed when the lists are built): eight lanes each, sharing the
+// listed candidates and adding their forces to the bond sum in the reference's order (extra_lanes).
+__global__ void __launch_bounds__(128) k_contact64(const __grid_constant__ DevView v) {
+  constexpr int L = 8;
+  const uint32_t nx = v.xcount[0];
+  const uint32_t sub = threadIdx.x & (L - 1), first = (threadIdx.x & 31u) - sub;
+  for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) / L; i < nx; i += gridDim.x * blockDim.x / L) {
+    const uint64_t n = v.xnodes[i];
+    const uint32_t k = v.pid[n];
+    const DevPart &P = v.parts[k];
+    const DevSimParams &sp = v.sp[P.sim];
+    DevSimState &st = v.ss[P.sim];
+    if (!st.active) continue;  // the group's lanes together
+    const D3 vi = ld3(v.vel_in, n, v.Ncap);
+    const ExtraCtx c = ctx64(v, n, k, P, sp, ld3(v.pos, n, v.Ncap), ld3(v.disp, n, v.Ncap), vi);
+    D3 f = ld3(v.force, n, v.Ncap);
+    if (v.cand_n[n] != kCandCells) f = extra_lanes<L>(v, n, P, sp, st, c, f, sub, first);
+    else if (sub == 0) f = extra_walk(v, n, P, sp, st, c, f);  // the cell walk: one lane
+    if (sub == 0) correct64(v, n, k, P, sp, st, vi, f);
   }
 }
 
@@ -354,7 +311,11 @@ void launch_step_kernel(const DevView &v, int precision, int variant, cudaStream
     return;
   }
   if (v.M) k_pair64<<<(unsigned)((v.M + 255) / 256), 256, 0, s>>>(v);
-  k_step<<<(unsigned)blocks, 128, 0, s>>>(v);
+  // a small handle's warps one to a block, so that they spread over every SM (8,338 nodes in blocks of
+  // 128 threads would use 66 of 152)
+  if (v.N < 152 * 512) k_step<<<(unsigned)((v.N + 31) / 32), 32, 0, s>>>(v);
+  else k_step<<<(unsigned)blocks, 128, 0, s>>>(v);
+  k_contact64<<<152 * 4, 128, 0, s>>>(v);
 }
 
 // ------------------------------------------------------------------------------------
