@@ -96,7 +96,8 @@ def build_engine(verbose: bool = False) -> Path:
                                [u for u in EXE_UNITS if (CSRC / u[0]).exists()]))
     lib = LIBDIR / LIBNAME
     if _stale(lib, objs):
-        cmd = [nvcc, *ARCH, "-shared", "-o", str(lib), *map(str, objs)]
+        # nodelete: the host pool's threads may still sleep in the library when a program closes it
+        cmd = [nvcc, *ARCH, "-shared", "-Xlinker", "-z", "-Xlinker", "nodelete", "-o", str(lib), *map(str, objs)]
         r = subprocess.run(cmd, capture_output=True, text=True)
         if r.returncode != 0:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")

@@ -31,6 +31,7 @@ inline uint64_t round_up(uint64_t x, uint64_t m) { return (x + m - 1) / m * m; }
 Engine::~Engine() {
   if (stream_) cudaStreamSynchronize(stream_);
   if (h_stage_) cudaFreeHost(h_stage_);
+  for (cudaEvent_t e : stage_ev_) cudaEventDestroy(e);
   for (int i = 0; i < 2; ++i)
     if (graph_[i]) cudaGraphExecDestroy(graph_[i]);
   for (void *p : allocs_) cudaFreeAsync(p, capture_stream_);
@@ -1310,14 +1311,14 @@ int Engine::sync(int timeout_ms) {
       err = "pd_sync: work still queued";
       return PD_ETIMEOUT;
     }
-    if (timeout_ms > 0) {
-      auto ms = std::chrono::duration_cast<std::chrono::milliseconds>(std::chrono::steady_clock::now() - t0).count();
-      if (ms > timeout_ms) {
-        err = "pd_sync: timed out after " + std::to_string(timeout_ms) + " ms";
-        return PD_ETIMEOUT;
-      }
+    const auto waited = std::chrono::steady_clock::now() - t0;
+    if (timeout_ms > 0 && waited > std::chrono::milliseconds(timeout_ms)) {
+      err = "pd_sync: timed out after " + std::to_string(timeout_ms) + " ms";
+      return PD_ETIMEOUT;
     }
-    std::this_thread::sleep_for(std::chrono::microseconds(50));
+    // a sleep overshoots by 50-100 us, several times a small handle's step: poll for the first
+    // millisecond
+    if (waited > std::chrono::milliseconds(1)) std::this_thread::sleep_for(std::chrono::microseconds(50));
   }
   DevCounters c;
   PD_TRY(cpy(&c, d_cnt_, sizeof(c), "read counters"));
@@ -1349,6 +1350,41 @@ void Engine::rows_to_file(const double *src, uint64_t stride, uint64_t node0, ui
   });
 }
 
+int Engine::read_staged(const double *src, double *dst, uint64_t n) {
+  // A copy straight into the caller's (pageable, often untouched) array runs at a few GB/s. Each host
+  // thread copies chunks into a pinned slot of its own and from there into the array, so that the
+  // copies of some chunks overlap the filling of others.
+  const uint64_t chunk = std::min(kStageChunk, std::max<uint64_t>(n / host_width(~0ull), 1ull << 15));
+  const uint64_t chunks = (n + chunk - 1) / chunk;
+  const unsigned width = host_width(std::max<uint64_t>(chunks, 1));
+  while (stage_ev_.size() < width) {
+    cudaEvent_t e;
+    PD_TRY(check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "staging event"));
+    stage_ev_.push_back(e);
+  }
+  // (the handle's reads all have the same size)
+  if (!h_stage_ && cudaMallocHost((void **)&h_stage_, width * chunk * 8) != cudaSuccess) {
+    cudaGetLastError();
+    h_stage_ = nullptr;
+    PD_TRY(check(cudaMemcpyAsync(dst, src, n * 8, cudaMemcpyDeviceToHost, stream_), "read state"));
+    return check(cudaStreamSynchronize(stream_), "read state");
+  }
+  int dev = 0;
+  PD_TRY(check(cudaGetDevice(&dev), "device"));
+  std::atomic<int> bad(cudaSuccess);
+  parallel_slots(chunks, [&](uint64_t i, unsigned slot) {
+    const uint64_t a = i * chunk, m = std::min(n - a, chunk);
+    double *stage = h_stage_ + slot * chunk;
+    cudaError_t e = cudaSetDevice(dev);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(stage, src + a, m * 8, cudaMemcpyDeviceToHost, stream_);
+    if (e == cudaSuccess) e = cudaEventRecord(stage_ev_[slot], stream_);
+    if (e == cudaSuccess) e = cudaEventSynchronize(stage_ev_[slot]);
+    if (e == cudaSuccess) std::memcpy(dst + a, stage, m * 8);
+    else bad = e;
+  });
+  return check((cudaError_t)bad.load(), "read state");
+}
+
 int Engine::get_state(double *curpos, double *vel, double *acc, double *force, double *disp) {
   PD_TRY(check(cudaStreamSynchronize(stream_), "sync"));
   // each array put in file order on the device, then copied straight to the caller
@@ -1360,12 +1396,6 @@ int Engine::get_state(double *curpos, double *vel, double *acc, double *force, d
   const bool fused = precision_ == PD_FP32C;
   const double *dcur = fused ? d_dispb_[cur_ ^ 1] : d_disp_;
   const uint32_t *clist = n_clamped_ ? d_clamped_ + (P_ + 1) : nullptr;
-  // Large handles copy through a pinned staging buffer and fill the caller's (pageable) arrays
-  // from it on all host cores: a pageable device-to-host copy runs at a few GB/s.
-  if (N_ >= kPinnedStageNodes && !h_stage_ && cudaMallocHost((void **)&h_stage_, 3 * N_ * 8) != cudaSuccess) {
-    cudaGetLastError();
-    h_stage_ = nullptr;
-  }
   int rc = PD_OK;
   auto out = [&](const double *src, const double *add, int clamped_mode, double *dst) {
     if (!dst || rc != PD_OK) return;
@@ -1374,15 +1404,11 @@ int Engine::get_state(double *curpos, double *vel, double *acc, double *force, d
     if (clamped_mode == 2)
       launch_clamped_rows(clist, n_clamped_, d_file_of_, d_pos_, d_clamped_disp_, Ncap_, rows, stream_);
     rc = check(cudaGetLastError(), "read state");
-    double *to = h_stage_ ? h_stage_ : dst;
-    if (rc == PD_OK) rc = check(cudaMemcpyAsync(to, rows, 3 * N_ * 8, cudaMemcpyDeviceToHost, stream_), "read state");
-    if (rc == PD_OK) rc = check(cudaStreamSynchronize(stream_), "read state");
-    if (rc == PD_OK && h_stage_) {
-      const uint64_t n = 3 * N_, chunk = 1ull << 17;  // 1 MB per item
-      parallel_items((n + chunk - 1) / chunk, [&](uint64_t i) {
-        const uint64_t a = i * chunk, b = std::min(n, a + chunk);
-        std::memcpy(dst + a, h_stage_ + a, (b - a) * 8);
-      });
+    if (rc == PD_OK && N_ >= kPinnedStageNodes) {
+      rc = read_staged(rows, dst, 3 * N_);
+    } else if (rc == PD_OK) {
+      rc = check(cudaMemcpyAsync(dst, rows, 3 * N_ * 8, cudaMemcpyDeviceToHost, stream_), "read state");
+      if (rc == PD_OK) rc = check(cudaStreamSynchronize(stream_), "read state");
     }
   };
   const bool stepped = steps_done_ > 0 && n_clamped_;

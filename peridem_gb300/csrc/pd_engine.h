@@ -40,27 +40,10 @@
 #include <thread>
 #include <vector>
 
+#include "pd_hostpool.h"
 #include "peridem_gb300.h"
 
 namespace pdg {
-
-// Runs f(i) for i in [0, n) on the host's cores (work handed out one index at a time).
-template <class F>
-void parallel_items(uint64_t n, F f) {
-  const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
-  const unsigned T = (unsigned)std::min<uint64_t>(std::min(hw, 32u), n);
-  if (T <= 1) {
-    for (uint64_t i = 0; i < n; ++i) f(i);
-    return;
-  }
-  std::atomic<uint64_t> next(0);
-  std::vector<std::thread> th;
-  for (unsigned t = 0; t < T; ++t)
-    th.emplace_back([&] {
-      for (uint64_t i = next++; i < n; i = next++) f(i);
-    });
-  for (auto &x : th) x.join();
-}
 
 constexpr int kSlice = 32;
 constexpr int kTileNodes = 256;           // nodes per block of the tiled bond kernel
@@ -576,7 +559,11 @@ class Engine {
   DevCounters *d_cnt_ = nullptr;
   uint32_t *d_clamped_ = nullptr;  // [P+1] offsets followed by engine node indices
   double *d_clamped_disp_ = nullptr;
-  double *h_stage_ = nullptr;  // pinned host staging of state reads on large handles (3 N doubles)
+  // pinned host staging of state reads on large handles: a chunk per host thread, and an event each
+  double *h_stage_ = nullptr;
+  std::vector<cudaEvent_t> stage_ev_;
+  // Device -> host copy of n doubles through the staging, ordered on the stream after what is queued.
+  int read_staged(const double *src, double *dst, uint64_t n);
   uint64_t n_clamped_ = 0;
   double *d_afd_ = nullptr;
   bool pv_possible_ = false, reset_possible_ = false;
@@ -591,7 +578,8 @@ class Engine {
 // size one thread per node already gives every SM ~27 warps, which hide the loads' latency.
 constexpr uint64_t kWarpCandNodes = 1ull << 17;
 // Handles of at least this many nodes read their state back through pinned host memory.
-constexpr uint64_t kPinnedStageNodes = 1ull << 18;
+constexpr uint64_t kPinnedStageNodes = 1ull << 17;
+constexpr uint64_t kStageChunk = 1ull << 17;  // doubles per copy at most (1 MB; 256 KB ones cost 3.98 M nodes 13 ms, 1 MB 10)
 
 // Arguments of the persistent step (k_persist, pd_fp32c.cu): the views of the two buffer
 // parities, the steps to run and the broad phase's buffers.
