@@ -250,7 +250,11 @@ struct BroadPhase {
   uint32_t *cand = nullptr;
   uint16_t *cand_n = nullptr;
   uint32_t cand_cap = 0;
-  double skin_frac = 0.5;
+  // contact skin over contact radius: the lists are rebuilt when nodes may have moved half of it. 0.6 instead
+  // of 0.5: the two-sphere impact 46 -> 32 rebuilds in 100 steps, 35.9 -> 32.9 us per step; packings within
+  // their noise. From 0.8 on the candidate radius reaches the nearest lattice neighbours (h - jitter for
+  // a radius of h / 2) and every node has candidates: crush 221 -> 268 us, cubes 36.7 -> 39.7
+  double skin_frac = 0.6;
   // the nodes that have contact candidates (rebuilt with the lists), in the FP32 form the particles
   // that need FP64 non-bond work next step, and their counts ([0] nodes, [1] particles)
   uint32_t *xnodes = nullptr, *xparts = nullptr, *xcount = nullptr;
