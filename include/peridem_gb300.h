@@ -232,12 +232,12 @@ int pd_close(pd_sim *sim);
  * candidates walks the broad phase's cell list instead, and after a pd_sync that saw one the
  * next pd_step doubles the capacity, up to 64), threads per block (<= 0 keeps it), per-step
  * statistics on/off (< 0 keeps it; on adds the pair-count kernel), step launch mode
- * (< 0 keeps it; 0 separate launches, 1 one CUDA graph per step, the FP64 default below 131,072
+ * (< 0 keeps it; 0 separate launches, 1 one CUDA graph per step, the FP64 default below 262,144
  * nodes, 2 the same graph with the broad-phase rebuild kernels in a conditional node, the
  * default above: fewer launches per step, but the conditional node itself costs a few
  * microseconds, which small handles feel; 3 all steps of a pd_step call in persistent
  * cooperative launches of one block per SM (up to 1024 steps each), the FP32C default below
- * 131,072 nodes, for handles without reset_partzero_y, prescribed-velocity or torque particles
+ * 163,840 nodes, for handles without reset_partzero_y, prescribed-velocity or torque particles
  * and with statistics off -- others step as in mode 2. A persistent launch occupies every SM
  * while it runs: handles stepping concurrently on other streams wait for it, so small handles
  * that step at the same time (a server's cohorts) should use mode 1. Its grid barriers wait at

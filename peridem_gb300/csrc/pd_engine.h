@@ -57,11 +57,16 @@ constexpr uint32_t kColBroken = 0x80000000u;  // FP32 form: broken flag in a col
 constexpr uint32_t kColIndex = 0x7FFFFFFFu;   // the partner index in a column entry
 constexpr uint64_t kOrderWindow = 1024;     // nodes per window of the bond-count sort (order_nodes)
 constexpr uint64_t kOrderWindow32 = 256;    // FP32 form, particles above kOrderWindow nodes: one tile's worth
-// FP32 handles of at least this many nodes (1024 tiles, 2.2 times the 456 resident at once) get the
-// tile arrays when they are created and step with the tiled bond kernel by default. Below, the
-// last, partly filled round of tiles costs more than the tiles save (200k nodes in contact: 98 us
-// against 84 us with the gather-ahead kernel 25; 363k: 121 against 145).
-constexpr uint64_t kTileMinNodes = 1ull << 18;
+// FP32 handles below this many nodes step in persistent launches; from it on they get the tile arrays
+// when they are created and step with the tiled bond kernel by default. Per step, persistent / tiled
+// in a step graph, us: a packing of 87k nodes 57 / 56, 139k 64 / 68, 196k 90 / 84, 248k 113 / 102; a
+// plate of 74k nodes 55 / 82, 143k 80 / 84, 213k 108 / 112; 83k nodes in contact 65 / 87, 201k 125 / 120
+// (tiles come 456 at a time, so the last, partly filled round weighs on handles of few rounds).
+constexpr uint64_t kPersistNodes = 163840;
+constexpr uint64_t kTileMinNodes = kPersistNodes;
+// From this many nodes on, the step graph holds the broad phase in a conditional node (213k nodes: 119 us
+// with it, 112 without; 248k: 104 and 102; the kernels it skips grow with the nodes).
+constexpr uint64_t kCondNodes = 1ull << 18;
 // From this many nodes on, the tiled kernel leaves the non-bond work to k_extra32 (778k nodes: 197 us
 // either way, 3.98 M: 935 against 961 us fused; 363k in contact: 132 against 121 us).
 constexpr uint64_t kTileSplitNodes = 1ull << 21;
