@@ -1054,7 +1054,8 @@ int Engine::alloc_and_upload() {
     cur_ = 1;
     PD_TRY(prepare_fused(cur_));
     if (N_ >= kTileMinNodes) {
-      PD_TRY(prepare_tiles());
+      PD_TRY(try_tiles());
+      if (!tiles_ready_) variant_ = 18;  // no room: the kernel that needs none
       // tiles that gather from global memory run slower than the plain kernel's: use that one where
       // they are common (horizons far wider than three node spacings)
       if (10ull * tiles_gathering_ > (N_ + kTileNodes - 1) / kTileNodes) variant_ = 18;
@@ -1970,6 +1971,25 @@ int Engine::prepare_tiles() {
   return PD_OK;
 }
 
+int Engine::try_tiles() {
+  const int rc = prepare_tiles();
+  if (rc != PD_ENOMEM) return rc;
+  err.clear();
+  const uint64_t nt = (N_ + kTileNodes - 1) / kTileNodes;
+  auto drop = [&](void *p, uint64_t bytes) {
+    if (!p) return;
+    cudaFreeAsync(p, capture_stream_);
+    device_bytes_ -= bytes;
+    allocs_.erase(std::remove(allocs_.begin(), allocs_.end(), p), allocs_.end());
+  };
+  drop(d_tile_rec_, nt * kTileRecords * 4);
+  drop(d_tile_n_, nt * 4);
+  drop(d_tcol_, std::max<uint64_t>(E_, 1) * 2);
+  d_tile_rec_ = d_tile_n_ = nullptr;
+  d_tcol_ = nullptr;
+  return PD_OK;
+}
+
 int Engine::refresh_tiles(bool tiled) {
   if (!tiles_ready_) return PD_OK;
   if (tiled && tiles_stale_) {
@@ -1996,7 +2016,7 @@ int Engine::set_variant(int variant) {
     return PD_EINVAL;
   }
   variant_ = variant;
-  if (tile_variant()) PD_TRY(prepare_tiles());
+  if (tile_variant()) PD_TRY(try_tiles());  // without room for the tiles it steps as variant 18
   graphs_ok_ = false;
   return PD_OK;
 }
@@ -2004,7 +2024,7 @@ int Engine::set_variant(int variant) {
 int Engine::autotune(uint32_t steps_per_variant, int *chosen, double *variant_ms) {
   const int nv = precision_ == PD_FP32C ? num_bond_variants() : 1;
   if (steps_per_variant == 0) steps_per_variant = 8;
-  if (nv > kFirstTileVariant) PD_TRY(prepare_tiles());
+  if (nv > kFirstTileVariant) PD_TRY(try_tiles());
   PD_TRY(snapshot());
   int best = variant_;
   double best_ms = 1e300;

@@ -462,6 +462,7 @@ class Engine {
   // FP32 form: the tile arrays of the tiled bond kernel, built on the device the first time they
   // are needed (at creation from kTileMinNodes nodes on).
   int prepare_tiles();
+  int try_tiles();  // prepare_tiles, but without device room gives back what it took and succeeds
   // Before steps are launched: the tile columns' broken flags follow the masks if other kernels have
   // stepped since the tiled one last did.
   int refresh_tiles(bool tiled);
