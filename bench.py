@@ -500,14 +500,13 @@ def ours(args):
         v64 = sum_over_ranks(dist, K64 * 0.5 * (l0 + l1)) / (ms64 * 1e-3)
         ph64 = sim64.profile(3) / 3
         ach64 = (4.125 * sim64.live_bonds() + 224.0 * s.n_nodes) / (ph64[2] * 1e-3) / 1e9
-        # FP64 add + multiply + fused multiply-add thread instructions per directed bond of
-        # k_step, counted by ncu on crush512 (sass_thread_inst_executed_op_{dadd,dmul,dfma}:
-        # 3.41e9 per launch, 7.52e7 bonds)
-        ops_per_bond = 45.4
+        # FP64 add / multiply / fma thread instructions per directed bond: half of k_pair64's 39 (each
+        # bond once, profiles/k_pair64_crush.md) and k_step's 7
+        ops_per_bond = 26.5
         fp64 = {"value": v64, "unit": UNIT, "steps": K64, "ms_per_step": ms64 / K64,
                 "kernel_ms": ph64[2], "roofline_hbm_frac": ach64 / peak,
                 "fp64_ops_per_s": v64 * ops_per_bond, "fp64_ops_per_bond": ops_per_bond,
-                "note": "bound by the FP64 issue rate (sqrt, reciprocal and divisions per bond), not HBM"}
+                "note": "bound by the FP64 issue rate (square root, reciprocal and divisions, once per bond), not HBM"}
         # accuracy of FP32C vs FP64 after the same number of steps on this workload
         done64 = W + K64 + 3
         if steps32 > done64:
@@ -596,7 +595,9 @@ def ours(args):
         "parallelism": "replicas" if world > 1 else "1 GPU",
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "traffic": traffic, "peak_source": peak_src,
-                     "kernel": f"k_extra32 + k_bond32 (variant {variant})", "kernel_ms": ph[2],
+                     "kernel": f"{'' if fused else 'k_extra32 + '}"
+                               f"{'k_bond32t' if 10 <= variant <= 13 else 'k_bond32'} (variant {variant})",
+                     "kernel_ms": ph[2],
                      "autotune_ms_per_variant": [round(float(x), 4) for x in variant_ms],
                      "phase_ms": {"predict": ph[0], "broadphase": ph[1], "step": ph[2], "end": ph[3]}},
         "cpu_baseline": cpu, "e2e": e2e, "fp64": fp64, "accuracy_vs_fp64": acc,
