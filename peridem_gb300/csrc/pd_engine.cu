@@ -864,8 +864,11 @@ int Engine::alloc_and_upload() {
   // FP32 form: each particle's records are relative to an anchor node, the node nearest the
   // centre of the particle's box (the FP32 rounding of a record grows with its distance from the
   // anchor); ext_p bounds the reference positions' rounding (set_break_band). xi_min is measured
-  // on the device once the bonds are built.
+  // on the device once the bonds are built. A checkpoint's records are relative to the anchor of the
+  // handle that saved it, so nodes equally near (a lattice symmetric about its centre) are ranked by the
+  // checkpoint's node order (ckpt_order), not by the order this engine keeps them in.
   std::atomic<bool> vol_varies(false);  // inside some particle
+  const uint32_t deg_bin = precision_ == PD_FP32C ? 16u : 1u;
   parallel_items(P_, [&](uint64_t k) {
     DevPart &P = parts[k];
     double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
@@ -874,6 +877,12 @@ int Engine::alloc_and_upload() {
         lo[c] = std::min(lo[c], pos[c * C + g]);
         hi[c] = std::max(hi[c], pos[c * C + g]);
       }
+    auto earlier = [&](uint32_t x, uint32_t y) {
+      const uint32_t fx = file_of_[x], fy = file_of_[y];
+      const uint64_t wx = (fx - P.g0) / kOrderWindow, wy = (fy - P.g0) / kOrderWindow;
+      const uint32_t bx = deg_file_[fx] / deg_bin, by = deg_file_[fy] / deg_bin;
+      return wx != wy ? wx < wy : bx != by ? bx > by : fx < fy;
+    };
     double best = INFINITY;
     uint32_t a = P.g0;
     for (uint64_t g = P.g0; g < (uint64_t)P.g0 + P.n; ++g) {
@@ -882,7 +891,7 @@ int Engine::alloc_and_upload() {
         const double d = pos[c * C + g] - 0.5 * (lo[c] + hi[c]);
         d2 += d * d;
       }
-      if (d2 < best) {
+      if (d2 < best || (d2 == best && earlier((uint32_t)g, a))) {
         best = d2;
         a = (uint32_t)g;
       }

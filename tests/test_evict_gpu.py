@@ -11,7 +11,7 @@ and gradient extforce (toggles), and a prescribed-velocity particle with reset_p
 import numpy as np
 import pytest
 
-from peridem_gb300 import _capi
+from peridem_gb300 import _capi, gen
 from peridem_gb300.sim import Batch, Sim
 from tests import cases
 
@@ -87,3 +87,28 @@ def test_a_finished_simulation_cannot_be_saved():
     assert e.value.rc == _capi.PD_ESTATE
     assert len(b.save_sim(1)) > 0
     b.close()
+
+
+@pytest.mark.parametrize("numbering", ["up", "down", "random"])
+def test_anchor_of_a_symmetric_lattice_follows_the_checkpoint_order(numbering):
+    """The eight nodes around the centre of an even lattice are equally near it; the records of a
+    checkpoint are relative to the one that comes first in the checkpoint's node order (windows of
+    1024 nodes of the file by descending bond count / 16), in whatever order the engine keeps the
+    nodes. A handle that chose another one would continue a saved simulation with its walls and
+    boxes shifted."""
+    h = 2.0 ** -13  # coordinates and distances without rounding
+    ax = (np.arange(16) - 7.5) * h
+    pos = np.stack(np.meshgrid(ax, ax, ax, indexing="ij"), axis=-1).reshape(-1, 3)
+    if numbering == "down":
+        pos = pos[::-1].copy()
+    elif numbering == "random":
+        pos = pos[np.random.default_rng(3).permutation(len(pos))]
+    s = gen.finish([gen.make_particle(pos, h, gen.GLASS, 3.0, np.random.default_rng(0), 0.0, (0, 0, 0))], 0.5 * h, 1e-8)
+    deg = np.bincount(s.conn.ravel(), minlength=len(pos))
+    order = sorted(range(len(pos)), key=lambda f: (f // 1024, -(int(deg[f]) // 16), f))
+    d2 = (s.pos ** 2).sum(axis=1)
+    first = next(f for f in order if d2[f] == d2.min())
+    sim = Sim(s, gen.base_config(1e-8, 10), "fp32c")
+    blob = sim.save_sim(0)
+    tail = len(blob) - 8 * len(sim.connectivity(0)) - 64  # the particle's fixed part, before its live pairs
+    np.testing.assert_array_equal(np.frombuffer(blob[tail + 16:tail + 40]), s.pos[first])
