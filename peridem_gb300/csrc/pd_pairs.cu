@@ -254,9 +254,12 @@ __device__ __forceinline__ bool visit(const PairsArgs &a, const Rec &me, F &&f) 
   return false;
 }
 
-// Every j > i of node i's particle within r; WRITE selects pass 1 (count) or 2 (write).
+// Every j > i of node i's particle within r; WRITE selects pass 1 (count) or 2 (write). A call with a
+// non-finite position is refused and none of its nodes searched: the box of such a particle may have
+// no finite corner, which puts all its nodes in one cell.
 template <bool WRITE>
 __global__ void k_pairs(PairsArgs a) {
+  if (*a.bad) return;
   for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < a.N; t += (uint64_t)gridDim.x * blockDim.x) {
     const Rec me = a.rec[t];
     const uint32_t base = (uint32_t)a.off[me.p];
@@ -277,6 +280,7 @@ __global__ void k_pairs(PairsArgs a) {
 // the reference's test: d = sqrt((dx*dx + dy*dy) + dz*dz), d <= r (gen_nonlocal_boundry_nodes,
 // exp_dict.py:1231-1248, which scans every node for every edge node).
 __global__ void k_near(PairsArgs a, const uint8_t *marked, uint8_t *near) {
+  if (*a.bad) return;  // as k_pairs
   for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < a.N; t += (uint64_t)gridDim.x * blockDim.x) {
     const Rec me = a.rec[t];
     near[me.node] = marked[me.node] || visit<true>(a, me, [&](const Rec &q) { return marked[q.node] != 0; });

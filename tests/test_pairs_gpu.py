@@ -7,6 +7,8 @@ scipy's compiled distance loop is platform code: x86 builds evaluate that expres
 written (checked here on 80,000 pairs within 3 ulps of r), while aarch64 builds contract it
 into fused multiply-adds, which moves pairs lying within an ulp of r. Against scipy, a pair may
 therefore differ only if its squared distance is within 4 ulps of r*r."""
+import time
+
 import numpy as np
 import pytest
 
@@ -180,3 +182,18 @@ def test_non_finite_position_is_refused():
     P[2, 1] = np.nan
     with pytest.raises(RuntimeError, match="non-finite"):
         gen.bonds_gpu([P], [1e-4])
+
+
+@pytest.mark.parametrize("bad", [-np.inf, np.inf, np.nan, -np.nan])
+def test_non_finite_position_is_refused_without_a_search(bad):
+    """-inf and a NaN with its sign bit set become the lower corner of the particle's box, and no node
+    has a cell then: the search, quadratic with every node in one cell (1.6e11 pairs here, seconds),
+    must not start."""
+    P = np.random.default_rng(1).uniform(0, 1e-2, (400000, 3))
+    gen.bonds_gpu([P[:8]], [1e-4])
+    P[12345, 1] = bad
+    for call in (lambda: gen.bonds_gpu([P], [1e-4]), lambda: gen.near_gpu([P], [np.zeros(len(P), bool)], [1e-4])):
+        t0 = time.perf_counter()
+        with pytest.raises(RuntimeError, match="non-finite"):
+            call()
+        assert time.perf_counter() - t0 < 0.5
