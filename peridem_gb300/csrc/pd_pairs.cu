@@ -218,7 +218,8 @@ __device__ __forceinline__ bool visit(const PairsArgs &a, const Rec &me, F &&f) 
   const float rc2 = (float)((r / c) * (r / c));
   float in2 = rc2 * (1.0f - 8e-6f), out2 = rc2 * (1.0f + 8e-6f);  // squared: within 4e-6 of r
   // FP64 decides everything where a box has more cells than FP32 in-cell positions are good for, or
-  // where r * r is near the ends of the FP64 range
+  // where r * r is near the ends of the FP64 range (a box wider than that range has NaN in-cell
+  // positions: the comparisons below let a NaN pass to FP64)
   bool wide = !(r2 > 1e-280 && r2 < 1e280);
   for (int d = 0; d < 3; ++d)
     wide = wide || !(val_of(a.hi[3 * (uint64_t)me.p + d]) - val_of(a.lo[3 * (uint64_t)me.p + d]) < 1e6 * c);
@@ -241,7 +242,7 @@ __device__ __forceinline__ bool visit(const PairsArgs &a, const Rec &me, F &&f) 
       if (q.cy != cy || q.cz != cz || q.p != me.p || dx < -1 || dx > 1 || q.node == me.node) continue;
       const float x = (float)dx + (q.fx - me.fx), y = q.fy + by, z = q.fz + bz;
       const float d2 = x * x + y * y + z * z;
-      if (!(d2 <= out2)) continue;
+      if (d2 > out2) continue;
       if (!(d2 < in2)) {  // too close to r for FP32
         const double *pi = a.pos + 3 * (uint64_t)me.node, *pj = a.pos + 3 * (uint64_t)q.node;
         const double ex = pj[0] - pi[0], ey = pj[1] - pi[1], ez = pj[2] - pi[2];

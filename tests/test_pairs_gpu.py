@@ -197,3 +197,13 @@ def test_non_finite_position_is_refused_without_a_search(bad):
         with pytest.raises(RuntimeError, match="non-finite"):
             call()
         assert time.perf_counter() - t0 < 0.5
+
+
+def test_box_wider_than_the_fp64_range():
+    """Coordinates whose difference overflows: nodes at one place are still within r of each other."""
+    P = np.zeros((5, 3))
+    P[[0, 2, 4]], P[[1, 3]] = 1e308, -1e308
+    m = np.array([0, 0, 1, 0, 0], dtype=bool)
+    with np.errstate(over="ignore"):
+        np.testing.assert_array_equal(gen.bonds_gpu([P], [1e150])[0], _formula(P, 1e150))
+        np.testing.assert_array_equal(gen.near_gpu([P], [m], [1e150])[0], _near_formula(P, m, 1e150))
