@@ -1384,25 +1384,28 @@ int Engine::read_staged(const double *src, double *dst, uint64_t n) {
     PD_TRY(check(cudaMemcpyAsync(dst, src, n * 8, cudaMemcpyDeviceToHost, stream_), "read state"));
     return check(cudaStreamSynchronize(stream_), "read state");
   }
-  const uint64_t chunk = std::min(kStageChunk, std::max<uint64_t>(n / host_width(~0ull), 1ull << 15));
-  const uint64_t chunks = (n + chunk - 1) / chunk;
-  const unsigned width = host_width(std::max<uint64_t>(chunks, 1));
-  while (stage_ev_.size() < width) {
+  // the slots are laid out once, for the threads there were then (the handle's reads all have the same
+  // size); a later read takes no more threads than it has slots
+  if (!h_stage_) {
+    stage_width_ = host_width(~0ull);
+    stage_chunk_ = std::min(kStageChunk, std::max<uint64_t>(n / stage_width_, 1ull << 15));
+    if (cudaMallocHost((void **)&h_stage_, stage_width_ * stage_chunk_ * 8) != cudaSuccess) {
+      cudaGetLastError();
+      h_stage_ = nullptr;
+      PD_TRY(check(cudaMemcpyAsync(dst, src, n * 8, cudaMemcpyDeviceToHost, stream_), "read state"));
+      return check(cudaStreamSynchronize(stream_), "read state");
+    }
+  }
+  while (stage_ev_.size() < stage_width_) {
     cudaEvent_t e;
     PD_TRY(check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "staging event"));
     stage_ev_.push_back(e);
   }
-  // (the handle's reads all have the same size)
-  if (!h_stage_ && cudaMallocHost((void **)&h_stage_, width * chunk * 8) != cudaSuccess) {
-    cudaGetLastError();
-    h_stage_ = nullptr;
-    PD_TRY(check(cudaMemcpyAsync(dst, src, n * 8, cudaMemcpyDeviceToHost, stream_), "read state"));
-    return check(cudaStreamSynchronize(stream_), "read state");
-  }
+  const uint64_t chunk = stage_chunk_, chunks = (n + chunk - 1) / chunk;
   int dev = 0;
   PD_TRY(check(cudaGetDevice(&dev), "device"));
   std::atomic<int> bad(cudaSuccess);
-  parallel_slots(chunks, [&](uint64_t i, unsigned slot) {
+  parallel_slots(chunks, stage_width_, [&](uint64_t i, unsigned slot) {
     const uint64_t a = i * chunk, m = std::min(n - a, chunk);
     double *stage = h_stage_ + slot * chunk;
     cudaError_t e = cudaSetDevice(dev);

@@ -571,6 +571,8 @@ class Engine {
   double *d_clamped_disp_ = nullptr;
   // pinned host staging of state reads on large handles: a chunk per host thread, and an event each
   double *h_stage_ = nullptr;
+  unsigned stage_width_ = 0;  // slots, of stage_chunk_ doubles each
+  uint64_t stage_chunk_ = 0;
   std::vector<cudaEvent_t> stage_ev_;
   // Device -> host copy of n doubles through the staging, ordered on the stream after what is queued.
   int read_staged(const double *src, double *dst, uint64_t n);

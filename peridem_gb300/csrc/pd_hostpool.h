@@ -125,11 +125,12 @@ inline unsigned host_width(uint64_t n) {
   return (unsigned)std::min<uint64_t>(std::min(hw, HostPool::kMax + 1), n);
 }
 
-// Runs f(i, slot) for i in [0, n) on the host's cores, work handed out one index at a time; slot <
-// host_width(n) tells the threads apart.
+// Runs f(i, slot) for i in [0, n) on up to `width` threads, work handed out one index at a time; slot <
+// max(width, 1) tells the threads apart. (The width is the caller's: the number of online cores, and
+// with it host_width, may change from one call to the next.)
 template <class F>
-void parallel_slots(uint64_t n, F f) {
-  const unsigned T = host_width(n);
+void parallel_slots(uint64_t n, unsigned width, F f) {
+  const unsigned T = (unsigned)std::min<uint64_t>(std::min(width, HostPool::kMax + 1), n);
   if (T <= 1) {
     for (uint64_t i = 0; i < n; ++i) f(i, 0u);
     return;
@@ -143,7 +144,7 @@ void parallel_slots(uint64_t n, F f) {
 // Runs f(i) for i in [0, n) on the host's cores.
 template <class F>
 void parallel_items(uint64_t n, F f) {
-  parallel_slots(n, [&](uint64_t i, unsigned) { f(i); });
+  parallel_slots(n, host_width(n), [&](uint64_t i, unsigned) { f(i); });
 }
 
 }  // namespace pdg
