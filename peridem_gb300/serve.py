@@ -131,8 +131,9 @@ class Server:
         self._est: dict = {}
 
     # -- admission ------------------------------------------------------------------------
-    def _pick(self, waiting: deque, est: dict) -> list:
-        """First fit in arrival order; a request whose cohort failed to build is retried alone."""
+    def _pick(self, waiting: deque, est: dict) -> tuple[list, int]:
+        """First fit in arrival order, and the bytes to reserve for it; a request whose cohort failed to
+        build is retried alone."""
         free = self.capacity - self.used
         pick, tot = [], 0
         for r in list(waiting):
@@ -145,7 +146,16 @@ class Server:
                 tot += b
                 if alone:
                     break
-        return pick
+        # A handle may hold more than its members would alone: from a certain size on it has the tiled
+        # bond kernel's arrays (about a quarter more). Where that could matter the cohort is estimated as
+        # one handle (12 ms of host work for 400k nodes) and its last requests wait.
+        while len(pick) > 1 and 4 * tot > free:
+            tot = max(tot, int(self.estimate([r.setup for r in pick], self.precision)))
+            if tot <= free:
+                break
+            pick.pop()
+            tot = sum(est[r.rid] for r in pick)
+        return pick, tot
 
     def _create(self, reqs: list, out: dict):
         t0 = time.perf_counter()
@@ -305,11 +315,10 @@ class Server:
                             waiting.appendleft(r)
             # start an admission
             if admit is None and waiting:
-                pick = self._pick(waiting, est)
+                pick, reserved = self._pick(waiting, est)
                 if pick:
                     for r in pick:
                         waiting.remove(r)
-                    reserved = sum(est[r.rid] for r in pick)
                     self.used += reserved
                     self.peak_used = max(self.peak_used, self.used)
                     out: dict = {}

@@ -228,3 +228,26 @@ def test_compaction_frees_finished_members_memory():
     res2 = srv2.run(reqs, realtime=False)
     assert not [e for e in srv2.log if e[1] == "evict"]
     assert [r.state["steps"] for r in res2] == [q.steps for q in reqs]
+
+
+def test_cohort_that_takes_more_than_its_members_respects_the_budget():
+    """A handle from 3000 nodes on takes a quarter more than its members would alone (as handles with
+    the tiled bond kernel's arrays do): what is reserved and held stays within the budget, and no
+    request waits for room that it does not need."""
+
+    def estimate(setups, precision):
+        n = sum(len(s.pos) for s in setups)
+        return n * BYTES_PER_NODE * 5 // (4 if n >= 3000 else 5)
+
+    class Larger(FakeBatch):
+        def __init__(self, setups, configs, precision):
+            super().__init__(setups, configs, precision)
+            self.nb = estimate(setups, precision)
+
+    FakeBatch.instances.clear()
+    cap = 4500 * BYTES_PER_NODE
+    srv = serve.Server("fp32c", capacity_bytes=cap, make_batch=Larger, estimate=estimate, chunk_steps=10)
+    res = srv.run([_req(i, 1000, 40) for i in range(8)], realtime=False)
+    assert all(r.error is None for r in res)
+    assert srv.peak_used <= cap and srv.used == 0
+    assert max(b.n for b in FakeBatch.instances) == 3  # four would take 5000 nodes' bytes
