@@ -391,12 +391,11 @@ __device__ __forceinline__ void verlet_tail(const DevView &v, uint64_t nn, uint3
       an = d3(0.0, 0.0, 0.0);
     }
     // predictor of the next step (timeloop.h:537-540)
-    D3 dn, inc;
+    D3 dn;
     if (clamped) {
       dn = d3(0.0, 0.0, 0.0);
-      inc = d;  // its length counts
     } else {
-      inc = sp.dt * vo + sp.hdt2 * an;
+      const D3 inc = sp.dt * vo + sp.hdt2 * an;
       dn = d + inc;
     }
     st3(v.force, nn, C3, f);
@@ -408,7 +407,8 @@ __device__ __forceinline__ void verlet_tail(const DevView &v, uint64_t nn, uint3
     st3(v.vel_out, nn, C3, vo);
     st3(v.disp_next, nn, C3, dn);
     set_rec_u(v.rec_next[nn], narrow(dn.x - anchor.x), narrow(dn.y - anchor.y), narrow(dn.z - anchor.z));
-    const float ix = magnitude(inc.x), iy = magnitude(inc.y), iz = magnitude(inc.z);
+    // how far it moves: with the rounding of d + inc, which may double an increment near d's last bit
+    const float ix = magnitude(dn.x - d.x), iy = magnitude(dn.y - d.y), iz = magnitude(dn.z - d.z);
     i2 = ix * ix + iy * iy + iz * iz;
   }
   // particle AABB of this step's positions in the particle's local frame, reduced over the warp as

@@ -10,6 +10,7 @@ per-launch step limit."""
 import numpy as np
 import pytest
 
+from peridem_gb300 import gen
 from peridem_gb300.sim import Batch, Sim
 from tests import cases
 
@@ -210,3 +211,21 @@ def test_autotune_may_pick_the_persistent_step():
     _compare(a, b, s.n_particles, "autotuned")
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("graphs", [1, 3])
+def test_movement_bound_includes_the_rounding_of_the_displacement(graphs):
+    """A node displaced by 1 whose increments are 0.6 of its last bit moves a whole bit every step: the
+    contact lists are rebuilt by what the nodes move, not by the increments alone."""
+    ulp = np.spacing(1.0)
+    s = gen.finish([gen.make_particle(np.zeros((1, 3)), 1e-4, gen.GLASS, 3.0, np.random.default_rng(0), 0.0, (0, 0, 0))],
+                   0.5e-4, 1e-8)
+    s.disp[:, 0] = 1.0
+    s.vel[:, 0] = 0.6 * ulp / 1e-8
+    s.contact_radius = 100 * ulp
+    a = Sim(s, gen.base_config(1e-8, 100), "fp32c")
+    a.tune(skin_frac=0.2, graphs=graphs)  # rebuilt after half the skin: 10 bits
+    assert a.graph_mode() == graphs
+    a.step(100)
+    assert a.state()["disp"][0, 0] >= 1.0 + 99 * ulp
+    assert a.stats()["rebuilds"] >= 9
