@@ -90,7 +90,8 @@ def set_bond_builder(kind: str):
 
 def bonds_gpu(positions: list, radii: list) -> list:
     """Pair lists of several point sets in one GPU call (pd_query_pairs): for each set, the
-    sorted (i, j), i < j, with |x_i - x_j| <= r."""
+    sorted (i, j), i < j, with |x_i - x_j| <= r. The lists of several sets share one array: copy a
+    list that is to be kept without the others."""
     import ctypes as C
     from ._capi import lib, ptr
     L = lib()
@@ -102,17 +103,20 @@ def bonds_gpu(positions: list, radii: list) -> list:
     rad = np.ascontiguousarray(radii, dtype=np.float64)
     po = np.zeros(P + 1, dtype=np.uint64)
     # room for a lattice with a horizon of three spacings (54 pairs per node); where that is too
-    # little the call says how many pairs there are. Pages of `out` that no pair reaches are never touched
-    cap = 60 * len(pos) + 1024
-    out = np.empty((cap, 2), dtype=np.uint32)
-    rc = L.pd_query_pairs(ptr(pos), ptr(off), ptr(rad), P, ptr(out), cap, ptr(po))
-    if rc != 0 and int(po[-1]) > cap:
-        cap = int(po[-1])
-        out = np.empty((cap, 2), dtype=np.uint32)
-        rc = L.pd_query_pairs(ptr(pos), ptr(off), ptr(rad), P, ptr(out), cap, ptr(po))
+    # little the call says how many pairs there are, and without room for that much it is asked first.
+    # Pages of `out` that no pair reaches are never touched
+    try:
+        out = np.empty((60 * len(pos) + 1024, 2), dtype=np.uint32)
+    except MemoryError:
+        out = None
+    rc = L.pd_query_pairs(ptr(pos), ptr(off), ptr(rad), P, ptr(out), 0 if out is None else len(out), ptr(po))
+    if (rc == 0 and out is None) or (rc != 0 and out is not None and int(po[-1]) > len(out)):
+        out = np.empty((int(po[-1]), 2), dtype=np.uint32)
+        rc = L.pd_query_pairs(ptr(pos), ptr(off), ptr(rad), P, ptr(out), len(out), ptr(po))
     if rc != 0:
         raise RuntimeError(f"pd_query_pairs: [{rc}] {L.pd_pairs_error().decode()}")
-    return [out[int(po[p]):int(po[p + 1])] for p in range(P)]
+    out.resize((int(po[-1]), 2), refcheck=False)  # gives the rest back
+    return [out] if P == 1 else [out[int(po[p]):int(po[p + 1])] for p in range(P)]
 
 
 def bonds(pos: np.ndarray, delta: float) -> np.ndarray:

@@ -207,3 +207,21 @@ def test_box_wider_than_the_fp64_range():
     with np.errstate(over="ignore"):
         np.testing.assert_array_equal(gen.bonds_gpu([P], [1e150])[0], _formula(P, 1e150))
         np.testing.assert_array_equal(gen.near_gpu([P], [m], [1e150])[0], _near_formula(P, m, 1e150))
+
+
+def test_lists_without_room_for_the_guess(monkeypatch):
+    """The call reserves room for 60 pairs a node; where the machine does not give it, the pairs are
+    counted first. A single particle's list is an array of its own."""
+    P = np.random.default_rng(2).uniform(0, 1e-3, (300, 3))
+    want, empty = _formula(P, 2e-4), np.empty
+
+    def no_guess(shape, *a, **kw):
+        if shape == (60 * 300 + 1024, 2):
+            raise MemoryError
+        return empty(shape, *a, **kw)
+
+    got = gen.bonds_gpu([P], [2e-4])[0]
+    np.testing.assert_array_equal(got, want)
+    assert got.flags.owndata and got.flags.writeable and got.nbytes == want.nbytes
+    monkeypatch.setattr(np, "empty", no_guess)
+    np.testing.assert_array_equal(gen.bonds_gpu([P], [2e-4])[0], want)
