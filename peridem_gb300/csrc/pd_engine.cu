@@ -221,6 +221,7 @@ int Engine::init(std::vector<HostSim> &sims, int precision) {
       return PD_EINVAL;
     }
   }
+  bp_.skin_frac = contact_skin();
   PD_TRY(check(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking), "cudaStreamCreate"));
   own_stream_ = true;
   capture_stream_ = stream_;
@@ -489,6 +490,24 @@ int Engine::bond_counts(std::vector<uint32_t> &deg, std::vector<uint64_t> *rowpt
   for (uint64_t sl = 0; sl < nslices_; ++sl) h_slice_ptr_[sl + 1] += h_slice_ptr_[sl];
   E_ = h_slice_ptr_[nslices_];
   return PD_OK;
+}
+
+double Engine::contact_skin() const {
+  constexpr uint64_t kChunk = 65536;
+  double skin = kSkinMost;
+  for (const HostSim &s : sims_) {
+    const uint64_t n = s.node_offset[s.np];
+    if (!n) continue;
+    std::vector<double> least((n + kChunk - 1) / kChunk);
+    parallel_items(least.size(), [&](uint64_t c) {
+      const double *v = s.vol.data();
+      least[c] = *std::min_element(v + c * kChunk, v + std::min(n, (c + 1) * kChunk));
+    });
+    const double spacing = std::cbrt(*std::min_element(least.begin(), least.end()));
+    const double fits = kCandSpacings * spacing / s.Rc - 1.0;
+    if (!(fits >= skin)) skin = fits;
+  }
+  return skin > kSkinLeast ? skin : kSkinLeast;
 }
 
 int Engine::alloc_bond_arrays() {

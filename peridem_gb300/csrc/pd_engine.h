@@ -246,6 +246,16 @@ struct DevView {
   const double *clamped_disp;
 };
 
+// The contact skin's range, in contact radii, and the largest candidate radius it may lead to, in lattice
+// spacings (the cube root of the smallest nodal volume). A wider skin rebuilds the lists less often: at
+// 0.6 instead of 0.5 the two-sphere impact 32 instead of 46 times in 100 steps (35.9 -> 32.9 us per step),
+// packings within their noise. But from 0.87 spacings on the candidate radius reaches the nodes' own
+// lattice neighbours (jittered by 5 %), and every node has candidates. Skin 0.5 / 0.6, us per step, by
+// contact radius in spacings: a packing of 453k nodes 0.54 147 / 148, 0.56 149 / 175, 0.58 149 / 190,
+// 0.62 190 / 221; 64k nodes of cubes 0.54 37.1 / 36.8, 0.56 36.6 / 39.7, 0.6 40.1 / 44.0; a plate of 363k
+// nodes 0.5 155 / 148, 0.58 206 / 225, 0.62 247 / 284.
+constexpr double kSkinLeast = 0.5, kSkinMost = 0.6, kCandSpacings = 0.85;
+
 // Broad-phase scratch (hashed cell list).
 struct BroadPhase {
   uint32_t table_bits = 0;
@@ -255,11 +265,9 @@ struct BroadPhase {
   uint32_t *cand = nullptr;
   uint16_t *cand_n = nullptr;
   uint32_t cand_cap = 0;
-  // contact skin over contact radius: the lists are rebuilt when nodes may have moved half of it. 0.6 instead
-  // of 0.5: the two-sphere impact 46 -> 32 rebuilds in 100 steps, 35.9 -> 32.9 us per step; packings within
-  // their noise. From 0.8 on the candidate radius reaches the nearest lattice neighbours (h - jitter for
-  // a radius of h / 2) and every node has candidates: crush 221 -> 268 us, cubes 36.7 -> 39.7
-  double skin_frac = 0.6;
+  // contact skin over contact radius (Engine::contact_skin): the lists are rebuilt when nodes may have
+  // moved half of it
+  double skin_frac = kSkinLeast;
   // the nodes that have contact candidates (rebuilt with the lists), in the FP32 form the particles
   // that need FP64 non-bond work next step, and their counts ([0] nodes, [1] particles)
   uint32_t *xnodes = nullptr, *xparts = nullptr, *xcount = nullptr;
@@ -451,6 +459,7 @@ class Engine {
   // Bond counts per engine node (deg), h_deg_, h_slice_ptr_, E_, initial_bonds_, and the row
   // starts of a row-contiguous layout when rowptr is given.
   int bond_counts(std::vector<uint32_t> &deg, std::vector<uint64_t> *rowptr);
+  double contact_skin() const;  // the default skin of this handle's simulations
   int alloc_bond_arrays();  // device SELL arrays, slice_ptr and deg uploaded
   // Device build from a sorted Connectivity, after bond_counts (rowptr: its row starts);
   // fallback = true when its scratch does not fit.

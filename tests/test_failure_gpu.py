@@ -111,3 +111,20 @@ def test_short_candidate_lists_leave_fp32c_results_unchanged():
     for p in range(s.n_particles):
         np.testing.assert_array_equal(a.connectivity(p), b.connectivity(p))
     assert b.stats()["device_errors"] == 0
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32c"])
+@pytest.mark.parametrize("spacings", [0.5, 0.52, 0.55, 0.6, 0.63, 0.66])
+def test_default_skin_stays_short_of_the_lattice(spacings, precision):
+    """With a contact radius below two thirds of the spacing the default candidate radius does not
+    reach a node's own lattice neighbours (six of them: lists of two would grow)."""
+    h = 1e-4
+    loc = gen.lattice("cube", 8 * h, h)
+    s = gen.finish([gen.make_particle(loc, h, gen.GLASS, 3.0, np.random.default_rng(0), 0.0, (0, 0, 0))],
+                   spacings * h, 1e-8)
+    sim = Sim(s, gen.base_config(1e-8, 10), precision)
+    sim.tune(cand_cap=2, graphs=1)  # the persistent step allocates its barriers when it first runs
+    b0 = _bytes(sim)
+    for _ in range(3):
+        sim.step(1)
+    assert _bytes(sim) == b0
