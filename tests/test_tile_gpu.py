@@ -1,11 +1,15 @@
 """The tiled bond kernel (variants 10-13) against the plain one (18): the same bits, with equal and
 with varying nodal volumes, with horizons whose records do not fit a tile, at node counts around a
 tile's and a slice's edges, and when other kernels broke bonds between its steps."""
+import mmap
+
 import numpy as np
 import pytest
 
 from peridem_gb300 import gen
-from peridem_gb300.sim import Sim
+from peridem_gb300._capi import lib, ptr
+from peridem_gb300.sim import Batch, Sim, estimate_bytes
+from tests import cases
 
 pytestmark = pytest.mark.gpu
 MM = 1e-3
@@ -74,3 +78,74 @@ def test_other_kernels_between_tiled_steps():
     b.step(4)
     a.step(4)
     _same(a, b, 2)
+
+
+@pytest.mark.parametrize("name", ["impact_free", "toggles"])
+def test_every_variant_in_the_step_graph(name):
+    """Each bond-kernel variant stepping in the step graph (a small handle's default, the persistent step,
+    has a bond loop of its own): the same bits as variant 18 and as the default."""
+    s, cfg = cases.CASES[name]()
+
+    def run(v):
+        a = Sim(s, cfg, "fp32c")
+        if v is not None:
+            a.tune(graphs=1)
+            a.set_variant(v)
+            assert a.graph_mode() == 1
+        a.step(25)
+        return a
+
+    ref = run(18)
+    _same(ref, run(None), s.n_particles)
+    for v in range(lib().pd_num_variants()):
+        _same(ref, run(v), s.n_particles)
+
+
+def test_default_path_of_a_large_handle():
+    """Just above the size from which a handle has tiles when it is created: a packing in contact with its
+    walls and a breaking impact in one handle, stepped as it comes, as larger handles step (conditional
+    graph, variant 10) and in the persistent launch, against variant 18 -- with a member that finishes
+    on the way. The memory estimate includes the tiles, and state reads give the same into pages in
+    use and untouched ones."""
+    items = [gen.crush_contact(count=24), gen.two_sphere(R=1e-3, v=60.0, gap=0.1, seed=2)]
+    setups, cfgs = [s for s, _ in items], [c for _, c in items]
+    est = estimate_bytes(setups, "fp32c")
+
+    def run(graphs, variant):
+        b = Batch(setups, cfgs, "fp32c")
+        assert 163840 <= b.N < 1 << 18 and b.device_bytes() == est
+        if graphs:
+            b.tune(graphs=graphs)
+        else:
+            assert b.graph_mode() == 1
+        if variant:
+            b.set_variant(variant)
+        b.step(25)
+        mid = b.state()
+        b.finish(1)
+        b.step(10)
+        return b, mid
+
+    ref, want = run(1, 18)
+    n0 = [len(s.conn) for s in setups]
+    for graphs, variant in ((0, 0), (2, 10), (3, 0)):
+        b, mid = run(graphs, variant)
+        for k in want:
+            np.testing.assert_array_equal(mid[k], want[k], err_msg=k)
+        left = [0, 0]
+        for i in (0, 1):
+            x, y = b.sim_state(i), ref.sim_state(i)
+            for k in x:
+                np.testing.assert_array_equal(x[k], y[k], err_msg=f"{i} {k}")
+            for p in range(setups[i].n_particles):
+                c = b.sim_connectivity(i, p)
+                np.testing.assert_array_equal(c, ref.sim_connectivity(i, p))
+                left[i] += len(c)
+        assert left[1] < n0[1]  # bonds broke
+        b.close()
+    used = np.full((ref.N, 3), 7.0)
+    new = np.frombuffer(mmap.mmap(-1, ref.N * 24), dtype=np.float64).reshape(ref.N, 3)
+    for out in (new, used):
+        assert lib().pd_get_node_state(ref.h, ptr(out), None, None, None, None) == 0
+    np.testing.assert_array_equal(new, used)
+    ref.close()
