@@ -13,8 +13,8 @@ Printed (one JSON line, rank 0):
   value       FP32-compensated form, device-timed (CUDA events, K steps, inputs resident)
   fp64        the plain FP64 form (bit-exact with the reference's CPU code) on the same setup
   e2e         pd_create_from_arrays from host arrays + K steps + pd_get_state back to host
-  roofline    fused step kernel: algorithmic bytes (4.125 B/live bond + 224 B/node) per
-              launch / its CUDA-event duration, against MEASURED_PEAKS.json's HBM copy rate
+  roofline    bond kernel: its algorithmic bytes (224 B/node and 4.125 B/live bond, tiled 2 B and
+              the tiles' lists) / its CUDA-event duration, against MEASURED_PEAKS.json's HBM copy rate
   cpu_baseline  the CPU oracle (restatement of the reference's serial/MPI-round-robin path)
               on a bounded sample (the first 32 particles of the same packing)
   accuracy    FP32-compensated vs FP64 after the same number of steps
@@ -168,19 +168,20 @@ def measured_peak():
     return 6800.0, "fallback 6.8 TB/s"
 
 
-def ncu_traffic(workload: str, precision: str, live: int, nodes: int):
-    """Per-launch DRAM bytes of the fused step kernel from a committed ncu summary, scaled
-    from the captured case to this launch by bonds and nodes (traffic grows with both)."""
+def ncu_traffic(variant: int, live: int, nodes: int):
+    """Per-launch DRAM bytes of the FP32C bond kernel from a committed ncu summary, scaled from the
+    captured case to this launch by bonds and nodes (traffic grows with both); None for another
+    variant than the captured one."""
     p = ROOT / "profiles" / "k_step_traffic.json"
     if not p.exists():
         return None
     try:
         d = json.loads(p.read_text())
-        e = d.get(precision)
-        if not e:
+        e = d["fp32c"]
+        if e["variant"] != variant:
             return None
-        per = (e["dram_bytes"]) / (4.125 * e["live_bonds"] + 224.0 * e["nodes"])
-        return per * (4.125 * live + 224.0 * nodes)
+        per = e["dram_bytes"] / (e["bond_bytes"] * e["live_bonds"] + 224.0 * e["nodes"])
+        return per * (e["bond_bytes"] * live + 224.0 * nodes)
     except Exception:
         return None
 
@@ -393,8 +394,8 @@ def workload_config(name: str, s, cfg) -> dict:
     """The workload description both arms print as `config` (the same dict)."""
     return {"workload": name, "particles": s.n_particles, "nodes": s.n_nodes,
             "directed_bonds": s.n_bonds_directed, "dt": cfg["dt"],
-            "l2": f"inputs larger than L2 ({(s.n_bonds_directed * 4.125 + s.n_nodes * 224) / 1e9:.2f} GB "
-                  f"touched per step vs 0.13 GB L2)"}
+            "l2": f"inputs larger than L2 ({(s.n_bonds_directed * 2 + s.n_nodes * 224) / 1e9:.2f} GB "
+                  f"and more touched per step vs 0.13 GB L2)"}
 
 
 def reference_arm(args):
@@ -484,9 +485,11 @@ def ours(args):
     nprof = max(3, min(20, K))
     ph = sim.profile(nprof) / nprof
     live_p = sim.live_bonds()
-    bytes_alg = 4.125 * live_p + 224.0 * s.n_nodes
+    # what this variant's kernel cannot do without: 2 B per bond and the tiles' lists if it is tiled
+    # (10-13), else 4.125 B per bond; 224 B per node (pd_step_bytes counts the bonds of the setup)
+    bytes_alg = sim.step_bytes() - (2.0 if 10 <= variant <= 13 else 4.125) * (s.n_bonds_directed - live_p)
     achieved = bytes_alg / (ph[2] * 1e-3) / 1e9
-    traffic = ncu_traffic(args.workload, "fp32c", live_p, s.n_nodes)
+    traffic = ncu_traffic(variant, live_p, s.n_nodes)
     steps32 = W + K + nprof
 
     # ---- FP64 plain form on the same setup

@@ -247,7 +247,8 @@ int pd_set_tuning(pd_sim *sim, double skin_frac, uint32_t cand_cap, int threads_
 /* Clears the device error word after the caller has handled it. */
 int pd_clear_device_errors(pd_sim *sim);
 
-/* Algorithmic byte count of one step (4.125 B per live directed bond + 224 B per node). */
+/* Algorithmic byte count of one step: 224 B per node and per live directed bond 4.125 B, or with a
+ * tiled bond kernel (variants 10-13) 2 B, and 4 B per entry of the tiles' record lists. */
 double pd_step_bytes(const pd_sim *sim);
 /* Phase timing (the reference's per-block wall clock, timeloop.h:909-947, per kernel
  * phase): runs nsteps real steps as separate launches with CUDA events between phases and

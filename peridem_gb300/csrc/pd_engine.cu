@@ -1705,7 +1705,9 @@ int Engine::clear_device_errors() {
 }
 
 double Engine::step_bytes(uint64_t live) const {
-  return 4.125 * (double)live + 224.0 * (double)N_;
+  // the tiled kernel reads 16-bit column entries with the broken flag in them and the tiles' lists
+  const bool tiled = precision_ == PD_FP32C && tiles_ready_ && tile_variant();
+  return (tiled ? 2.0 : 4.125) * (double)live + (tiled ? 4.0 * (double)tile_records_ : 0.0) + 224.0 * (double)N_;
 }
 
 }  // namespace pdg
@@ -1992,8 +1994,10 @@ int Engine::prepare_tiles() {
   PD_TRY(cpy(cnt.data(), d_tile_n_, nt * 4, "read tiles"));
   tile_max_ = 0;
   tiles_gathering_ = 0;
+  tile_records_ = 0;
   for (uint32_t c : cnt) {
     tile_max_ = std::max(tile_max_, c);
+    tile_records_ += c;
     tiles_gathering_ += c == 0;
   }
   PD_TRY(check(prepare_tile_kernels(), "tile kernels"));

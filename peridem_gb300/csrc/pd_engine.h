@@ -566,6 +566,7 @@ class Engine {
   uint16_t *d_tcol_ = nullptr;
   uint32_t tile_max_ = 0;
   uint32_t tiles_gathering_ = 0;  // tiles whose records do not fit
+  uint64_t tile_records_ = 0;     // entries of all tiles' lists
   bool tile_vol_ = false;         // see DevView
   bool tiles_ready_ = false, tiles_stale_ = false;
   uint8_t *d_extra_flag_ = nullptr;

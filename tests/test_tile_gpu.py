@@ -149,3 +149,14 @@ def test_default_path_of_a_large_handle():
         assert lib().pd_get_node_state(ref.h, ptr(out), None, None, None, None) == 0
     np.testing.assert_array_equal(new, used)
     ref.close()
+
+
+def test_step_bytes_of_the_kernel_in_use():
+    s, cfg = _impact(900)
+    a = Sim(s, cfg, "fp32c")
+    nodes, tiles = 224.0 * s.n_nodes, -(-s.n_nodes // 256)
+    a.set_variant(18)
+    assert a.step_bytes() == 4.125 * s.n_bonds_directed + nodes
+    a.set_variant(10)
+    lists = a.step_bytes() - 2.0 * s.n_bonds_directed - nodes
+    assert 4 * s.n_nodes <= lists <= 4 * min(3072, s.n_nodes) * tiles
