@@ -21,11 +21,6 @@ __device__ __forceinline__ void st3(double *a, uint64_t n, uint64_t cap, D3 v) {
   a[n + 2 * cap] = v.z;
 }
 
-__device__ __forceinline__ double warp_max(double v) {
-  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
-}
-
 // intersects_box_fext<3> (contact.h:1143-1183): only box A is extended by c.
 __device__ __forceinline__ bool intersects_fext(const double *A, const double *B, double c) {
   double A_min_x = A[0] - c, A_min_y = A[1] - c, A_min_z = A[2] - c;

@@ -109,7 +109,6 @@ DevView Engine::view(int cur) const {
   v.pair = d_pair_;
   v.pidx = d_pidx_;
   v.plow = d_plow_;
-  v.E = E_;
   v.anchor = d_anchor_;
   if (precision_ == PD_FP32C) {
     v.disp = d_dispb_[cur];
@@ -120,7 +119,6 @@ DevView Engine::view(int cur) const {
     v.clamp_flag = d_clamp_flag_;
     v.fused = 1;
   }
-  v.break_band = 1e-4;
   v.f_extra = d_f_extra_;
   v.tile_rec = d_tile_rec_;
   v.tile_n = d_tile_n_;

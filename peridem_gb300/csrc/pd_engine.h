@@ -185,7 +185,6 @@ struct DevView {
   const uint16_t *deg;
   const uint32_t *col;
   uint32_t *mask;
-  uint64_t E;
   // FP64 form, the bonds as pairs (k_pair64): the owner and the partner of each of the M pairs, their
   // constants xi, |xi|, RN(1/|xi|) ([5][M]) and this step's terms; per SELL entry the pair it is, and
   // per (slice, position) the lanes whose entry is the partner's side
@@ -202,7 +201,6 @@ struct DevView {
   int fused;                  // 1: FP32 form with the fused predictor
   const double *anchor;       // [P][3] anchor of rec[].u (this step)
   double *anchor_next;        // [P][3] anchor of rec_next[].u
-  double break_band;     // relative band around snot where the FP64 stretch decides
   double *f_extra;       // [3][Ncap] FP64 non-bond force density of flagged nodes
   // FP32 form, tiled bond kernel (prepare_tiles): per tile of kTileNodes nodes, the list of the
   // distinct records its bonds read ([ntiles][kTileRecords], tile_n of them; 0: more than fit, the
