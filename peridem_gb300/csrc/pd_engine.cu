@@ -55,6 +55,9 @@ int Engine::raw_alloc(void **p, size_t bytes) {
     err = std::string("device allocation of ") + std::to_string(bytes) + " B: " + cudaGetErrorString(e);
     return e == cudaErrorMemoryAllocation ? PD_ENOMEM : PD_ECUDA;
   }
+  // the memory is ready in the order of the handle's own stream; work on a caller's stream may touch it
+  // next (tile arrays of a variant chosen later, the persistent step's barriers, a snapshot)
+  if (stream_ != capture_stream_) cudaStreamSynchronize(capture_stream_);
   device_bytes_ += bytes;
   return PD_OK;
 }

@@ -160,3 +160,28 @@ def test_step_bytes_of_the_kernel_in_use():
     a.set_variant(10)
     lists = a.step_bytes() - 2.0 * s.n_bonds_directed - nodes
     assert 4 * s.n_nodes <= lists <= 4 * min(3072, s.n_nodes) * tiles
+
+
+def test_tiles_built_on_a_callers_stream():
+    """The tile arrays are allocated when a variant first needs them, in the handle's own stream, and
+    built and read on the stream the caller chose meanwhile, beside another handle that does the same."""
+    torch = pytest.importorskip("torch")
+    s, cfg = _impact(900)
+    ref = Sim(s, cfg, "fp32c")
+    ref.tune(graphs=1)
+    ref.set_variant(18)
+    ref.step(16)
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    sims = [Sim(s, cfg, "fp32c") for _ in streams]
+    for a, q in zip(sims, streams):
+        a.set_stream(q.cuda_stream)
+        a.tune(graphs=1)
+        a.step(8, sync=False)
+    for a in sims:
+        a.set_variant(10)
+        a.step(8, sync=False)
+    for a in sims:
+        a.sync()
+        _same(a, ref, 2)
+        a.set_stream(None)
+        a.close()
