@@ -1085,9 +1085,12 @@ int Engine::alloc_and_upload() {
     if (N_ >= kTileMinNodes) {
       PD_TRY(try_tiles());
       if (!tiles_ready_) variant_ = 18;  // no room: the kernel that needs none
-      // tiles that gather from global memory run slower than the plain kernel's: use that one where
-      // they are common (horizons far wider than three node spacings)
-      if (10ull * tiles_gathering_ > (N_ + kTileNodes - 1) / kTileNodes) variant_ = 18;
+      // a tile whose records do not fit is stepped after the others, alone on its SM, and its rows are
+      // the longest: one of them costs more than the tiles save. Plain / tiled, us per step: 520k nodes
+      // with 3 such tiles 324 / 405, 2.1 M with 5 782 / 939; horizons of 4.75 spacings 512k (14 tiles)
+      // 553 / 605, of 5 216k (30) 316 / 362, 512k (161) 637 / 638; without such tiles, horizon 4.5,
+      // 512k 523 / 408
+      if (tiles_wide_) variant_ = 18;
     }
   }
   PD_TRY(check(cudaStreamSynchronize(stream_), "init sync"));
@@ -1995,11 +1998,15 @@ int Engine::prepare_tiles() {
   PD_TRY(cpy(cnt.data(), d_tile_n_, nt * 4, "read tiles"));
   tile_max_ = 0;
   tiles_gathering_ = 0;
+  tiles_wide_ = 0;
   tile_records_ = 0;
-  for (uint32_t c : cnt) {
+  for (uint64_t t = 0; t < nt; ++t) {
+    const uint32_t c = cnt[t];
     tile_max_ = std::max(tile_max_, c);
     tile_records_ += c;
     tiles_gathering_ += c == 0;
+    const uint64_t s0 = t * (kTileNodes / 32), s1 = std::min(s0 + kTileNodes / 32, nslices_);
+    tiles_wide_ += c == 0 && h_slice_ptr_[s1] > h_slice_ptr_[s0];  // it has bonds
   }
   PD_TRY(check(prepare_tile_kernels(), "tile kernels"));
   tiles_ready_ = true;

@@ -210,7 +210,7 @@ struct DevView {
   const uint32_t *tile_rec, *tile_n;
   uint16_t *tcol;
   uint32_t tile_max;     // longest list: the kernel's shared-memory size in records
-  uint32_t tile_gather;  // tiles whose records do not fit
+  uint32_t tile_gather;  // tiles without a list (no bonds, or too many records)
   int tile_vol;          // 1: records carry cnot * volume (it varies inside a particle), 0: one per particle
   // FP32 form: work lists of k_extra32 (see BroadPhase)
   uint32_t *xnodes, *xparts, *xcount;
@@ -563,7 +563,8 @@ class Engine {
   uint32_t *d_tile_rec_ = nullptr, *d_tile_n_ = nullptr;
   uint16_t *d_tcol_ = nullptr;
   uint32_t tile_max_ = 0;
-  uint32_t tiles_gathering_ = 0;  // tiles whose records do not fit
+  uint32_t tiles_gathering_ = 0;  // tiles without a list: without bonds, or more records than fit
+  uint32_t tiles_wide_ = 0;       // the latter
   uint64_t tile_records_ = 0;     // entries of all tiles' lists
   bool tile_vol_ = false;         // see DevView
   bool tiles_ready_ = false, tiles_stale_ = false;

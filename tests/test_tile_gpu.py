@@ -185,3 +185,29 @@ def test_tiles_built_on_a_callers_stream():
         _same(a, ref, 2)
         a.set_stream(None)
         a.close()
+
+
+@pytest.mark.parametrize("other", ["wide", "bondless"])
+def test_default_kernel_of_a_large_handle_by_its_tiles(other):
+    """Tiles are the default from 163,840 nodes on unless some tile's records do not fit; tiles without
+    bonds do not count. pd_step_bytes tells the kernels apart."""
+    h, rng = 0.1 * MM, np.random.default_rng(0)
+
+    def part(n, factor, x):
+        loc = gen.lattice("cube", n * h, h)
+        return gen.make_particle(loc, h, gen.GLASS, factor, rng, 0.05, (x * h, 0, 0))
+
+    gen.set_bond_builder("gpu")
+    try:
+        s = gen.finish([part(56, 2.0, 0.0), part(20, 6.0 if other == "wide" else 0.5, 60.0)], 0.5 * h, 1e-8)
+    finally:
+        gen.set_bond_builder("cpu")
+    a = Sim(s, gen.base_config(1e-8, 10), "fp32c")
+    plain = 4.125 * s.n_bonds_directed + 224.0 * s.n_nodes
+    assert a.step_bytes() == plain if other == "wide" else a.step_bytes() < plain
+    b = Sim(s, gen.base_config(1e-8, 10), "fp32c")
+    b.tune(graphs=1)
+    b.set_variant(12 if other == "wide" else 18)
+    a.step(3)
+    b.step(3)
+    _same(a, b, 2)
