@@ -297,7 +297,8 @@ void Engine::order_nodes(const std::vector<HostSim> &sims, std::vector<uint32_t>
   // counted on crush512_4m's particles 1,447 records per tile of 256 nodes at any alignment of
   // the tiles (windows of the file order: 2,407; recursive bisection, dearer to compute: 1,412), at
   // 1.09x padding with counts sorted in bins of 16. A particle of up to kOrderWindow nodes keeps
-  // its file order: its tiles read at most the particle's records in any order.
+  // its file order: its tiles read at most the particle's records in any order. So does one of more than
+  // kCurveBonds bonds a node, whose tiles do not fit in any order.
   // The order depends on the particle alone (a checkpoint moves between handles), and per-node
   // results do not depend on it: each node's sums keep the reference's row order, and every
   // sequence that the reference takes in node order (contact partners, particle means) is taken
@@ -343,7 +344,8 @@ void Engine::order_nodes(const std::vector<HostSim> &sims, std::vector<uint32_t>
     if (!srt) all_sorted = false;
     std::vector<uint32_t> along(nloc), idx(nloc);
     for (uint64_t k = 0; k < nloc; ++k) along[k] = (uint32_t)k;
-    const bool along_curve = spatial && nloc > kOrderWindow;
+    const uint64_t pairs = s.conn_offset[p + 1] - s.conn_offset[p];
+    const bool along_curve = spatial && nloc > kOrderWindow && 2 * pairs <= kCurveBonds * nloc;
     const uint64_t window = along_curve ? kOrderWindow32 : kOrderWindow;
     if (along_curve) morton_order(s.pos.data() + 3 * s.node_offset[p], s.vol.data() + s.node_offset[p], along);
     std::vector<uint32_t> hist;

@@ -56,6 +56,10 @@ constexpr uint32_t kMaxCandCap = 64;      // largest per-node candidate list
 constexpr uint32_t kColBroken = 0x80000000u;  // FP32 form: broken flag in a column entry
 constexpr uint32_t kColIndex = 0x7FFFFFFFu;   // the partner index in a column entry
 constexpr uint64_t kOrderWindow = 1024;     // nodes per window of the bond-count sort (order_nodes)
+// FP32 form: most bonds a node of a particle kept along a curve. Above it the tiles do not fit, and the plain
+// kernel gathers longer runs of the file's lattice order: horizons of 5.25, 6 and 7 spacings (557, 810 and
+// 1,220 bonds a node), 216k nodes: 330, 478 and 720 us a step against 357, 534 and 844 along the curve.
+constexpr uint64_t kCurveBonds = 500;
 constexpr uint64_t kOrderWindow32 = 256;    // FP32 form, particles above kOrderWindow nodes: one tile's worth
 // FP32 handles below this many nodes step in persistent launches; from it on they get the tile arrays
 // when they are created and step with the tiled bond kernel by default. Per step, persistent / tiled
@@ -411,7 +415,7 @@ class Engine {
   // descending bond count (stable: equal counts keep their file order). FP32 form: a particle of
   // more than kOrderWindow nodes along a Morton curve of cells of ~64 nodes (file order inside a
   // cell), then inside each window of kOrderWindow32 nodes by descending bond count / 16; smaller
-  // particles as the FP64 form, by count / 16. file_of[engine index] = file index, node_of = its inverse,
+  // particles and those of more than kCurveBonds bonds a node as the FP64 form, by count / 16. file_of[engine index] = file index, node_of = its inverse,
   // deg_file = bond count of each node in file order (indices out of range are not counted).
   static void order_nodes(const std::vector<HostSim> &sims, std::vector<uint32_t> &file_of,
                           std::vector<uint32_t> &node_of, std::vector<uint32_t> &deg_file,
