@@ -10,6 +10,7 @@ import numpy as np
 import pytest
 
 from oracle import oracle as O
+from peridem_gb300 import gen
 from peridem_gb300._capi import lib
 from peridem_gb300.sim import Sim
 from tests import cases
@@ -259,3 +260,29 @@ def test_damage_field(precision):
         orc = O.Oracle(s, cfg)
         orc.step(40)
         np.testing.assert_array_equal(d, O.damage(s, [orc.connectivity(p) for p in range(s.n_particles)]))
+
+
+@pytest.mark.parametrize("n", [1, 255, 256, 257, 512, 1300])
+def test_file_order_means_around_a_round_of_terms(n):
+    """The means of a particle with torque, of one with a prescribed velocity and of particle 0 when it is
+    put on top (reset_partzero_y) are sums in file node order, fetched 256 terms at a time: bit for bit
+    the oracle's at sizes around a round's edges and for a numbering far from the engine's order."""
+    rng = np.random.default_rng(n)
+    h = 1e-4
+    loc = gen.lattice("cube", 12 * h, h)
+    loc = loc[np.argsort((loc ** 2).sum(axis=1), kind="stable")[:n]]
+    loc = loc[rng.permutation(n)]
+    parts = [gen.make_particle(loc, h, gen.GLASS, 3.0, rng, 0.05, (k * 13 * h, 0, 0), vel=tuple(rng.uniform(-5, 5, 3)))
+             for k in range(2)]
+    s = gen.finish(parts, 0.5 * h, 1e-8)
+    s.torque_val[:] = [1e9, -2e9]
+    s.torque_axis[1] = 1
+    cfg = gen.base_config(1e-8, 12, set_torque_timestep=2, particle_w_fixed_velocity=0, set_fix_velocity_timestep=3,
+                          fix_velocity_mean_x=1, prescribed_velocity_mean_x=-2.5, fix_velocity_angular=1,
+                          prescribed_angular_vel=2.0e4, reset_partzero_y=1, reset_partzero_y_timestep=6,
+                          wheel_rad=15 * h)
+    sim, orc = Sim(s, cfg, "fp64"), O.Oracle(s, cfg)
+    for t in (4, 12):
+        sim.step(t - (0 if t == 4 else 4))
+        orc.step(t - (0 if t == 4 else 4))
+        _compare_exact("means", s, sim, orc, t)
