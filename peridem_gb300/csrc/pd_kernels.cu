@@ -282,25 +282,43 @@ __global__ void __launch_bounds__(128) k_step(DevView v) {
 }
 
 // The nodes with contact candidates (listed when the lists are built): eight lanes each, sharing the
-// listed candidates and adding their forces to the bond sum in the reference's order (extra_lanes).
+// listed candidates and adding their forces to the bond sum in the reference's order (extra_lanes). A
+// warp's four groups start each round of nodes together: once apart they stay so, and the warp takes
+// their nodes one after another (453k nodes with 29 candidates each: a few such warps 10 ms, all others 2).
+// Then the nodes whose list overflowed, a thread each in the engine's order, so that the threads of a warp
+// scan the same cells (453k nodes at a contact radius of 1.6 spacings, some of them: 26 ms a step with one of
+// the eight lanes, 19 now; of 1.9, all of them: 3.9 s, 1.2 now).
 __global__ void __launch_bounds__(128) k_contact64(const __grid_constant__ DevView v) {
-  constexpr int L = 8;
-  const uint32_t nx = v.xcount[0];
-  const uint32_t sub = threadIdx.x & (L - 1), first = (threadIdx.x & 31u) - sub;
-  for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) / L; i < nx; i += gridDim.x * blockDim.x / L) {
-    const uint64_t n = v.xnodes[i];
+  constexpr uint32_t L = 8, G = 32 / L;
+  const uint32_t nx = v.xcount[0], lane = threadIdx.x & 31u, sub = lane & (L - 1);
+  const uint32_t thread = blockIdx.x * blockDim.x + threadIdx.x, threads = gridDim.x * blockDim.x;
+  auto node = [&](uint64_t n, bool writer, auto add) {
     const uint32_t k = v.pid[n];
     const DevPart &P = v.parts[k];
     const DevSimParams &sp = v.sp[P.sim];
     DevSimState &st = v.ss[P.sim];
-    if (!st.active) continue;  // the group's lanes together
+    if (!st.active) return;
     const D3 vi = ld3(v.vel_in, n, v.Ncap);
     const ExtraCtx c = ctx64(v, n, k, P, sp, ld3(v.pos, n, v.Ncap), ld3(v.disp, n, v.Ncap), vi);
-    D3 f = ld3(v.force, n, v.Ncap);
-    if (v.cand_n[n] != kCandCells) f = extra_lanes<L>(v, n, P, sp, st, c, f, sub, first);
-    else if (sub == 0) f = extra_walk(v, n, P, sp, st, c, f);  // the cell walk: one lane
-    if (sub == 0) correct64(v, n, k, P, sp, st, vi, f);
+    const D3 f = add(P, sp, st, c, ld3(v.force, n, v.Ncap));
+    if (writer) correct64(v, n, k, P, sp, st, vi, f);
+  };
+  for (uint32_t i0 = thread / 32 * G; i0 < nx; i0 += threads / 32 * G) {
+    __syncwarp();
+    const uint32_t i = i0 + lane / L;
+    if (i >= nx) continue;  // the group's lanes together
+    const uint64_t n = v.xnodes[i];
+    if (v.cand_n[n] == kCandCells) continue;
+    node(n, sub == 0, [&](const DevPart &P, const DevSimParams &sp, DevSimState &st, const ExtraCtx &c, D3 f) {
+      return extra_lanes<L>(v, n, P, sp, st, c, f, sub, lane - sub);
+    });
   }
+  if (nx == 0) return;
+  for (uint64_t n = thread; n < v.N; n += threads)
+    if (v.cand_n[n] == kCandCells)
+      node(n, true, [&](const DevPart &P, const DevSimParams &sp, DevSimState &st, const ExtraCtx &c, D3 f) {
+        return extra_walk(v, n, P, sp, st, c, f);
+      });
 }
 
 void launch_step_kernel(const DevView &v, int precision, int variant, cudaStream_t s) {
