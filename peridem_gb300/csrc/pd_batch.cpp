@@ -174,10 +174,9 @@ int Engine::finish_sim(uint32_t sim) {
 
 // ---- per-simulation checkpoints (eviction and re-admission) ----------------------------
 //
-// A simulation's nodes occupy one contiguous engine range whose internal order depends only on
-// its own setup (order_nodes sorts inside each particle), and its particles one contiguous
-// range; so the simulation's slices of every per-node and per-particle array are copied as
-// they are. What depends on the handle -- global node indices in the bond columns and the
+// A simulation's nodes occupy one contiguous engine range, and its particles one contiguous
+// range; its slices of every per-particle array are copied as they are, those of the per-node
+// arrays in the checkpoint's node order (ckpt_order), which depends on its setup alone. What depends on the handle -- global node indices in the bond columns and the
 // SELL slices' live masks, the contact lists, the cell list, the work lists -- is not copied:
 // the live bonds travel as each particle's Connectivity and the rest is rebuilt by the next
 // step. The FP32 form's two displacement buffers, records and velocity buffer are saved by

@@ -132,7 +132,7 @@ __device__ __forceinline__ void bp_candidates_node(const DevView &v, uint64_t t,
   } else {
     cand_n[me.node] = (uint16_t)cnt;
   }
-  if (v.xnodes) v.xnodes[atomicAdd(&v.xcount[0], 1u)] = me.node;  // FP32 form: work list
+  if (v.xnodes) v.xnodes[atomicAdd(&v.xcount[0], 1u)] = me.node;  // work list of the contact kernels
 }
 
 // Words of shared memory bp_candidates_quad takes per warp: four gather buffers of kMaxCandCap

@@ -3,8 +3,10 @@
 // Layout in HBM (all particles of all simulations of a batch concatenated in file order; the
 // nodes of particle p occupy the engine indices [node_offset[p], node_offset[p+1]) as in the
 // file, but inside each window of kOrderWindow of them they are sorted by descending bond
-// count (stable), so that the 32 rows of a SELL slice have nearly equal lengths; node_of /
-// file_of map the two numberings and every host-facing array is in file order):
+// count (stable), so that the 32 rows of a SELL slice have nearly equal lengths -- in the FP32
+// form larger particles first along a Morton curve, so that a tile's nodes lie together
+// (order_nodes); node_of / file_of map the two numberings and every host-facing array is in
+// file order):
 //   * node state, FP64 structure-of-arrays: pos/disp/vel/acc/force/extforce as [3][Ncap]
 //     (x block, y block, z block), vol[N]; vel is double-buffered (the fused kernel reads
 //     partners' step-start velocity while it writes the corrected one);
