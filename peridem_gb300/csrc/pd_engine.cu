@@ -242,19 +242,39 @@ int Engine::init(std::vector<HostSim> &sims, int precision) {
 
 
 // Sorts along (0 .. n-1 on entry) by the Morton code of each node's cell, keeping file order inside
-// a cell. Cells hold ~64 nodes of the particle's mean nodal volume; at most 1024 of them a side.
+// a cell. Cells hold ~64 nodes of the particle's mean nodal volume; at most 1024 of them a side. Chunks of
+// nodes on the host's cores (one large particle would wait for one of them: 512k nodes 7.5 ms), of a
+// fixed size, so that the sum of the volumes does not depend on the cores.
 static void morton_order(const double *pos, const double *vol, std::vector<uint32_t> &along) {
-  const uint64_t n = along.size();
-  double lo[3] = {pos[0], pos[1], pos[2]}, hi[3] = {pos[0], pos[1], pos[2]}, vsum = 0;
-  for (uint64_t k = 0; k < n; ++k) {
-    for (int c = 0; c < 3; ++c) {
-      lo[c] = std::min(lo[c], pos[3 * k + c]);
-      hi[c] = std::max(hi[c], pos[3 * k + c]);
+  constexpr uint64_t kChunk = 32768;
+  const uint64_t n = along.size(), nc = (n + kChunk - 1) / kChunk;
+  struct Part {
+    double lo[3], hi[3], vsum = 0;
+    uint32_t all = 0;  // bits set in some key
+  };
+  std::vector<Part> part(nc);
+  parallel_items(nc, [&](uint64_t x) {
+    Part a;
+    for (int c = 0; c < 3; ++c) a.lo[c] = a.hi[c] = pos[3 * x * kChunk + c];
+    for (uint64_t k = x * kChunk; k < std::min(n, (x + 1) * kChunk); ++k) {
+      for (int c = 0; c < 3; ++c) {
+        a.lo[c] = std::min(a.lo[c], pos[3 * k + c]);
+        a.hi[c] = std::max(a.hi[c], pos[3 * k + c]);
+      }
+      a.vsum += vol[k];
     }
-    vsum += vol[k];
+    part[x] = a;
+  });
+  Part all = part[0];
+  for (uint64_t x = 1; x < nc; ++x) {
+    for (int c = 0; c < 3; ++c) {
+      all.lo[c] = std::min(all.lo[c], part[x].lo[c]);
+      all.hi[c] = std::max(all.hi[c], part[x].hi[c]);
+    }
+    all.vsum += part[x].vsum;
   }
-  const double ext = std::max(std::max(hi[0] - lo[0], hi[1] - lo[1]), hi[2] - lo[2]);
-  const double cell = std::max(std::cbrt(64.0 * vsum / (double)n), ext / 1023.0), inv = 1.0 / cell;
+  const double ext = std::max(std::max(all.hi[0] - all.lo[0], all.hi[1] - all.lo[1]), all.hi[2] - all.lo[2]);
+  const double cell = std::max(std::cbrt(64.0 * all.vsum / (double)n), ext / 1023.0), inv = 1.0 / cell;
   if (!(cell > 0) || !std::isfinite(inv) || !std::isfinite(ext)) return;  // no geometry to go by
   auto spread = [](uint32_t x) {  // ten bits, two zero bits between them
     x = (x | (x << 16)) & 0x030000FFu;
@@ -263,22 +283,30 @@ static void morton_order(const double *pos, const double *vol, std::vector<uint3
     return (x | (x << 2)) & 0x09249249u;
   };
   std::unique_ptr<uint32_t[]> key(new uint32_t[n]);
-  uint32_t all = 0;
-  for (uint64_t k = 0; k < n; ++k) {
-    uint32_t m = 0;
-    for (int c = 0; c < 3; ++c) {
-      const double q = (pos[3 * k + c] - lo[c]) * inv;
-      m |= spread(q >= 0 ? (uint32_t)std::min(q, 1023.0) : 0u) << c;
+  parallel_items(nc, [&](uint64_t x) {
+    uint32_t bits = 0;
+    for (uint64_t k = x * kChunk; k < std::min(n, (x + 1) * kChunk); ++k) {
+      uint32_t m = 0;
+      for (int c = 0; c < 3; ++c) {
+        const double q = (pos[3 * k + c] - all.lo[c]) * inv;
+        m |= spread(q >= 0 ? (uint32_t)std::min(q, 1023.0) : 0u) << c;
+      }
+      key[k] = m;
+      bits |= m;
     }
-    key[k] = m;
-    all |= m;
-  }
-  std::vector<uint32_t> to(n);
-  for (int sh = 0; sh < 30 && (all >> sh); sh += 10) {  // stable radix sort of the nodes by their keys
-    uint32_t at[1025] = {0};
-    for (uint64_t k = 0; k < n; ++k) at[((key[k] >> sh) & 1023u) + 1]++;
-    for (int d = 0; d < 1024; ++d) at[d + 1] += at[d];
-    for (uint64_t k = 0; k < n; ++k) to[at[(key[along[k]] >> sh) & 1023u]++] = along[k];
+    part[x].all = bits;
+  });
+  for (const Part &a : part) all.all |= a.all;
+  int bits = 0;  // of the largest key, in equal digits of at most 15 (32,768 cells, 2 M nodes, in one pass)
+  while (all.all >> bits) ++bits;
+  const int passes = (bits + 14) / 15, width = passes ? (bits + passes - 1) / passes : 0;
+  std::vector<uint32_t> to(n), at((1ull << width) + 1);
+  for (int sh = 0; sh < bits; sh += width) {  // stable radix sort of the nodes by their keys
+    auto digit = [&](uint64_t k) { return (key[k] >> sh) & ((1u << width) - 1u); };
+    std::fill(at.begin(), at.end(), 0u);
+    for (uint64_t k = 0; k < n; ++k) at[digit(k) + 1]++;
+    for (uint32_t d = 0; d < 1u << width; ++d) at[d + 1] += at[d];
+    for (uint64_t k = 0; k < n; ++k) to[at[digit(along[k])]++] = along[k];
     along.swap(to);
   }
 }
