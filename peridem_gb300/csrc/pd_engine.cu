@@ -376,26 +376,30 @@ void Engine::order_nodes(const std::vector<HostSim> &sims, std::vector<uint32_t>
     const bool along_curve = spatial && nloc > kOrderWindow && 2 * pairs <= kCurveBonds * nloc;
     const uint64_t window = along_curve ? kOrderWindow32 : kOrderWindow;
     if (along_curve) morton_order(s.pos.data() + 3 * s.node_offset[p], s.vol.data() + s.node_offset[p], along);
-    std::vector<uint32_t> hist;
-    for (uint64_t w0 = 0; w0 < nloc; w0 += window) {
-      const uint64_t w1 = std::min<uint64_t>(nloc, w0 + window);
-      auto bin = [&](uint64_t k) { return dg[along[k]] / deg_bin; };
-      uint32_t dmax = 0;
-      for (uint64_t k = w0; k < w1; ++k) dmax = std::max(dmax, bin(k));
-      if (dmax < 4096) {  // stable counting sort by descending count
-        hist.assign(dmax + 2, 0);
-        for (uint64_t k = w0; k < w1; ++k) hist[dmax - bin(k) + 1]++;
-        for (uint32_t d = 1; d <= dmax + 1; ++d) hist[d] += hist[d - 1];
-        for (uint64_t k = w0; k < w1; ++k) idx[w0 + hist[dmax - bin(k)]++] = along[k];
-      } else {
-        std::copy(along.begin() + w0, along.begin() + w1, idx.begin() + w0);
-        std::stable_sort(idx.begin() + w0, idx.begin() + w1, [&](uint32_t a, uint32_t b) { return dg[a] / deg_bin > dg[b] / deg_bin; });
+    constexpr uint64_t kChunk = 32 * kOrderWindow;  // whole windows, a large particle's on all cores
+    parallel_items((nloc + kChunk - 1) / kChunk, [&](uint64_t x) {
+      const uint64_t end = std::min<uint64_t>(nloc, (x + 1) * kChunk);
+      std::vector<uint32_t> hist;
+      for (uint64_t w0 = x * kChunk; w0 < end; w0 += window) {
+        const uint64_t w1 = std::min<uint64_t>(nloc, w0 + window);
+        auto bin = [&](uint64_t k) { return dg[along[k]] / deg_bin; };
+        uint32_t dmax = 0;
+        for (uint64_t k = w0; k < w1; ++k) dmax = std::max(dmax, bin(k));
+        if (dmax < 4096) {  // stable counting sort by descending count
+          hist.assign(dmax + 2, 0);
+          for (uint64_t k = w0; k < w1; ++k) hist[dmax - bin(k) + 1]++;
+          for (uint32_t d = 1; d <= dmax + 1; ++d) hist[d] += hist[d - 1];
+          for (uint64_t k = w0; k < w1; ++k) idx[w0 + hist[dmax - bin(k)]++] = along[k];
+        } else {
+          std::copy(along.begin() + w0, along.begin() + w1, idx.begin() + w0);
+          std::stable_sort(idx.begin() + w0, idx.begin() + w1, [&](uint32_t a, uint32_t b) { return dg[a] / deg_bin > dg[b] / deg_bin; });
+        }
       }
-    }
-    for (uint64_t k = 0; k < nloc; ++k) {
-      file_of[g0 + k] = (uint32_t)(g0 + idx[k]);
-      node_of[g0 + idx[k]] = (uint32_t)(g0 + k);
-    }
+      for (uint64_t k = x * kChunk; k < end; ++k) {
+        file_of[g0 + k] = (uint32_t)(g0 + idx[k]);
+        node_of[g0 + idx[k]] = (uint32_t)(g0 + k);
+      }
+    });
   });
   if (bad) *bad = bad_p.load();
   if (sorted) *sorted = all_sorted.load();
